@@ -381,13 +381,6 @@ __device__ __forceinline__ float neg_exp2i(uint32_t p) {  // 2^-p for p <= 126
     return (p == 0) ? 1.0f : bitsf((127u - p) << 23);
 }
 
-// The reference steps into an empty child, then on the next iteration
-// computes that child's exit, moves tMin past it and pops.  Here that pair
-// of iterations is one: the empty child's exit is computed in place.  The
-// corner moves by powers of two and stays exactly representable, so the
-// add/subtract pair of the reference changes nothing and the operations
-// that reach tMin are the same.  The voxel size test uses a per-level
-// table of the same products.
 // The descent that every cone from one origin shares.  At the start of a
 // trace, tMin moves only when a cone skips an empty child, so while the
 // point origin + dir * tMin lies on the same side of each centre plane for
@@ -409,6 +402,7 @@ struct ConePrefix {
     uint32_t depth;      // its level
     uint32_t stack;      // child ids on the way down, unmirrored, 3 bits each
     float corner[3];     // its minimum corner in the normalised frame
+    uint32_t path[10];   // the nodes on the way down, by level (path[0] the root)
     uint32_t termId;     // with `term`: the node every cone stops at
     uint32_t term;       // 1: every cone stops at termId
     uint32_t termLeaf;   // ... which is a leaf
@@ -460,6 +454,7 @@ __device__ __forceinline__ ConePrefix cone_prefix(const GuideDev& g, V3 pos, flo
         for (int a = 0; a < 3; a++)
             if ((c >> a) & 1u) corner[a] += half;
         stack = (stack << 3) | c;
+        P.path[level] = nodeId;
         nodeId = child;
         P.nodeId = nodeId;
         P.depth = lvl;
@@ -472,8 +467,8 @@ __device__ __forceinline__ ConePrefix cone_prefix(const GuideDev& g, V3 pos, flo
 }
 
 // The trace in two parts: cone_begin is the setup before the loop,
-// cone_step one iteration of it.  The Morton stack holds at
-// most leafDepth <= 10 levels of 3 bits.
+// cone_trace the loop.  The Morton stack holds at most leafDepth <= 10
+// levels of 3 bits.
 struct ConeState {
     V3 dc, pb, corner;
     float tMin;
@@ -540,90 +535,130 @@ __device__ __forceinline__ bool cone_begin(const GuideDev& g, V3 pos, V3 dir, fl
     return false;
 }
 
-// Per-level constants of the cone loop, computed once per block: span[L] =
-// 2^-L (neg_exp2i) and vs2[L] = the squared voxel size of level L
-// (level_voxel_size_sqr).  Same values as computing them in the loop.
-struct ConeTables {
-    const float* span;  // 12 entries (levels 0..11)
-    const float* vs2;   // 11 entries (levels 0..10)
+// What the cones of a block share in shared memory: vs2[L], the squared
+// voxel size of level L (level_voxel_size_sqr, 11 entries), and the ids of
+// the nodes on each thread's way down, entry L * stride for level L (levels
+// 0..9), at this thread's own column.
+struct ConeShared {
+    const float* vs2;
+    uint32_t* path;
+    uint32_t stride;
 };
 
-// One iteration of the reference's loop.  The empty-child skip takes the
-// child's exit crossings from values the iteration already has: per axis
-// the child's far plane is the node's far plane (child bit set: corner +
-// span/2 + span/2 = corner + span, exact for these dyadic corners) or its
-// centre plane, so the crossings are tm or tc, value for value.  True when
-// the trace has ended.
-__device__ __forceinline__ bool cone_step(const GuideDev& g, float aperture,
-                                          uint32_t maxQueryLevelOffset, ConeState& s,
-                                          bool& isLeaf, uint32_t& leafId,
-                                          const ConeTables* tab = nullptr) {
-    if (s.step == kConeTraceMaxSteps) {
-        leafId = kInvalid;
-        isLeaf = false;
-        return true;
-    }
-    s.step++;
-    const float childSpan = tab ? tab->span[s.depth + 1] : neg_exp2i(s.depth + 1);
-    const float curSpan = tab ? tab->span[s.depth] : neg_exp2i(s.depth);
-    const V3 topRight = s.corner + v3(curSpan, curSpan, curSpan);
-    const V3 tm = topRight * s.dc - s.pb;
-    const float tMax = fminf(fminf(tm.x, tm.y), tm.z);
-    const uint64_t node = g.nodes[s.nodeId];
-    if (tMax < s.tMin) {
-        const uint32_t b = s.stack & 7u;
-        s.corner = s.corner - v3((b & 1u) ? curSpan : 0.0f, (b & 2u) ? curSpan : 0.0f,
-                                 (b & 4u) ? curSpan : 0.0f);
-        s.stack >>= 3;
-        s.depth -= 1;
-        s.nodeId = svo_parent(node);
-        return s.nodeId == kSvoInvalidParent;  // left the tree: a miss
-    }
-    const V3 center = s.corner + v3(childSpan, childSpan, childSpan);
-    const V3 tc = center * s.dc - s.pb;
-    uint32_t childId = 0;
-    if (tc.x < s.tMin) childId |= 1u;
-    if (tc.y < s.tMin) childId |= 2u;
-    if (tc.z < s.tMin) childId |= 4u;
-    const uint32_t mir = childId ^ s.mirror;
-    if (!((svo_mask(node) >> mir) & 1u)) {
-        // empty child: leave it at once
-        const float ex = (childId & 1u) ? tm.x : tc.x;
-        const float ey = (childId & 2u) ? tm.y : tc.y;
-        const float ez = (childId & 4u) ? tm.z : tc.z;
-        s.tMin = next_up(fminf(fminf(ex, ey), ez));
-        return false;
-    }
-    const uint32_t child = svo_child_index(node) + svo_child_offset(node, mir);
-    const uint32_t level = s.depth + 1;
-    const float area = s.tMin * s.tMin * aperture;
-    const float diam2 = 4.0f * (area * kInvPiF);
-    bool term = diam2 > (tab ? tab->vs2[level] : level_voxel_size_sqr(g, level));
-    const bool childLeaf = svo_children_leaf(node);
-    term |= (g.leafDepth - level) <= maxQueryLevelOffset;
-    if (childLeaf || term) {
-        isLeaf = childLeaf;
-        leafId = child;
-        return true;
-    }
-    s.nodeId = child;
-    s.corner = s.corner + v3((childId & 1u) ? childSpan : 0.0f, (childId & 2u) ? childSpan : 0.0f,
-                             (childId & 4u) ? childSpan : 0.0f);
-    s.stack = (s.stack << 3) | childId;
-    s.depth = level;
-    return false;
-}
-
+// The trace.  The reference takes one iteration per event (a descent, the
+// step over an empty child, or the return to the parent), reading the node
+// and rebuilding its crossings in each.  Here, with the same values:
+//   - the crossings of the node's far planes (tm) and centre planes (tc) are
+//     kept.  An empty child is left in place: its exit is, per axis, the
+//     node's far plane (child bit set: corner + span/2 + span/2 = corner +
+//     span, exact for these dyadic corners) or its centre plane.  A child
+//     entered has those crossings as its far planes, none below tMin (a
+//     clear bit means tc >= tMin, and tm >= tMin held for the node), so only
+//     a skip can leave a node;
+//   - a skip returns to the ancestor it ends in at once.  The planes behind
+//     tMin are far planes of the node on some axes; an ancestor shares such
+//     a plane, and with it the crossing, for as long as the Morton bits of
+//     that axis are ones, and its far planes on the other axes lie no nearer
+//     than the node's (the products and differences round monotonically).
+//     So the reference pops at least one level more than the trailing ones
+//     of each such axis, and the crossings of the node found are tested as
+//     it tests them (the loop repeats should they still be behind tMin).
+// Corners are held as 1 + corner, in [1, 2), so that an ancestor's corner is
+// the mantissa cut to its level's bits.
+// Bound by instruction issue: the lanes of a warp are at different events
+// (Cornell 128x128, depth 1: 35.6 iterations per 32 cones, 18 lanes in each;
+// popping level by level ran 2.0 rounds of its loop per iteration for 4
+// lanes at a time, 40 % of the instructions).  The 64x64 fields of a frame:
+// 8.52 -> 7.99 ms there, 6.68 -> 6.25 ms on clusters-1M at 1920x1080.  Idle
+// lanes taking the next texels once 8, 16 or 24 of a warp's have ended cost
+// more than they gain (9.5, 9.9 and 10.1 ms): the lanes lose their coherence.
 __device__ __forceinline__ float cone_trace(const GuideDev& g, V3 pos, V3 dir, float tMin,
                                             float aperture, uint32_t maxQueryLevelOffset,
                                             bool& isLeaf, uint32_t& leafId,
-                                            const ConePrefix* pre = nullptr,
-                                            const ConeTables* tab = nullptr) {
+                                            const ConePrefix& pre, const ConeShared& sh) {
     ConeState s;
-    if (cone_begin(g, pos, dir, tMin, pre, s, isLeaf, leafId)) return s.tMin;
-    while (!cone_step(g, aperture, maxQueryLevelOffset, s, isLeaf, leafId, tab)) {
+    if (cone_begin(g, pos, dir, tMin, &pre, s, isLeaf, leafId)) return s.tMin;
+    const V3 dc = s.dc, pb = s.pb;
+    float t = s.tMin;
+    uint32_t stack = s.stack, depth = s.depth, step = s.step, nodeId = s.nodeId;
+    float cx = 1.0f + s.corner.x, cy = 1.0f + s.corner.y, cz = 1.0f + s.corner.z;
+    uint32_t shared = pre.depth;  // levels whose node is still the prefix's
+    float span = neg_exp2i(depth);
+    uint64_t node = __ldg(g.nodes + nodeId);
+    V3 tm;
+    float tMax;
+    auto far_planes = [&]() {
+        const float s1 = span - 1.0f;
+        tm = v3((cx + s1) * dc.x - pb.x, (cy + s1) * dc.y - pb.y, (cz + s1) * dc.z - pb.z);
+        tMax = fminf(fminf(tm.x, tm.y), tm.z);
+    };
+    far_planes();
+    // leave the nodes that end before t; false when the tree was left
+    auto pop = [&]() {
+        do {
+            constexpr uint32_t kAxis = 0x09249249u;  // every third bit
+            const uint32_t zeros = ~stack;
+            // 3 * (levels - 1) + 1 per axis whose far plane lies behind
+            uint32_t l = 1u;
+            if (tm.x < t) l = max(l, uint32_t(__ffs(int(zeros & kAxis))));
+            if (tm.y < t) l = max(l, uint32_t(__ffs(int((zeros >> 1) & kAxis))));
+            if (tm.z < t) l = max(l, uint32_t(__ffs(int((zeros >> 2) & kAxis))));
+            l += 2u;
+            const uint32_t levels = (l * 11u) >> 5;  // l / 3 for l <= 33
+            if (levels > depth) return false;
+            step += levels;
+            depth -= levels;
+            stack >>= l;
+            const uint32_t keep = 0xFFFFFFFFu << (23u - depth);
+            cx = __uint_as_float(__float_as_uint(cx) & keep);
+            cy = __uint_as_float(__float_as_uint(cy) & keep);
+            cz = __uint_as_float(__float_as_uint(cz) & keep);
+            span = neg_exp2i(depth);
+            node = __ldg(g.nodes + (depth < shared ? pre.path[depth]
+                                                   : sh.path[depth * sh.stride]));
+            shared = min(shared, depth + 1u);
+            far_planes();
+        } while (tMax < t);
+        return true;
+    };
+    sh.path[depth * sh.stride] = nodeId;
+    if (tMax < t && !pop()) return t;
+    while (step < kConeTraceMaxSteps) {
+        step++;
+        const float half = 0.5f * span, h1 = half - 1.0f;
+        const V3 tc = v3((cx + h1) * dc.x - pb.x, (cy + h1) * dc.y - pb.y, (cz + h1) * dc.z - pb.z);
+        const bool bx = tc.x < t, by = tc.y < t, bz = tc.z < t;
+        const uint32_t childId = (bx ? 1u : 0u) | (by ? 2u : 0u) | (bz ? 4u : 0u);
+        const uint32_t mir = childId ^ s.mirror;
+        const uint32_t mask = svo_mask(node);
+        // far planes of the child
+        const V3 te = v3(bx ? tm.x : tc.x, by ? tm.y : tc.y, bz ? tm.z : tc.z);
+        if (!((mask >> mir) & 1u)) {
+            t = next_up(fminf(fminf(te.x, te.y), te.z));
+            if (tMax < t && !pop()) return t;
+            continue;
+        }
+        const uint32_t child = svo_child_index(node) + __popc(mask & ((1u << mir) - 1u));
+        depth++;
+        const float area = t * t * aperture;
+        const float diam2 = 4.0f * (area * kInvPiF);
+        const bool childLeaf = svo_children_leaf(node);
+        if (childLeaf || diam2 > sh.vs2[depth] || (g.leafDepth - depth) <= maxQueryLevelOffset) {
+            isLeaf = childLeaf;
+            leafId = child;
+            return t;
+        }
+        node = __ldg(g.nodes + child);
+        sh.path[depth * sh.stride] = child;
+        if (bx) cx += half;
+        if (by) cy += half;
+        if (bz) cz += half;
+        stack = (stack << 3) | childId;
+        span = half;
+        tm = te;
+        tMax = fminf(fminf(te.x, te.y), te.z);
     }
-    return s.tMin;
+    return t;
 }
 
 // AnisoSVOctreeGPU::FindMarkedBin (AnisoSVO.cuh:1244-1262): walk up from
