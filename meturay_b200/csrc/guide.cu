@@ -947,8 +947,8 @@ uint32_t guide_launches(const SvoResult& v, const GuideOptions& go, uint32_t max
     const uint32_t D = static_cast<uint32_t>(v.levelOffsets.size()) - 2;
     const uint32_t collapse = 1 + (D > go.minBinLevel ? D - go.minBinLevel : 0);
     // memsets are not kernels; init, collapse, resolve, sort (histogram,
-    // scan, 4 onesweep passes), heads, scan (3), ranges, guide
-    return 1 + collapse + 1 + 6 + 1 + 3 + 1 + 1;
+    // 4 onesweep passes), heads, scan (3), ranges, guide
+    return 1 + collapse + 1 + 5 + 1 + 3 + 1 + 1;
 }
 
 int guide_wavefront(const SceneDev& sc, const GuideDev& g, const SvoResult& v, const GuideWave& w,

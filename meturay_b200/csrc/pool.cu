@@ -189,14 +189,10 @@ int record_iteration(mrb_pool* p) {
             return r;
         // also adds this wavefront to the traced-ray total and clears the
         // next wavefront's counter
-        if ((r = dense_keys(ho.key, cnt + cur, p->maxRays, p->idBits, p->dense.as<uint32_t>(), pt,
-                            st, p->counters.as<unsigned long long>(), cnt + nxt)))
-            return r;
-        if ((r = radix_sort_pairs<uint32_t>(p->dense.as<uint32_t>(), p->sortedIds.as<uint32_t>(),
-                                            cnt + cur, p->maxRays, 0, 3 + int(p->idBits), true,
-                                            p->sortTemp.p, p->sortTempBytes, st, true)))
-            return r;
-        if ((r = find_portions(p->dense.as<uint32_t>(), cnt + cur, p->maxRays, p->idBits, pt, st)))
+        if ((r = partition_rays(ho.key, cnt + cur, p->maxRays, p->idBits,
+                                p->sortedIds.as<uint32_t>(), p->dense.as<uint32_t>(), false, pt,
+                                p->sortTemp.p, p->sortTempBytes, st,
+                                p->counters.as<unsigned long long>(), cnt + nxt)))
             return r;
         const HitIn hi{ho.key, ho.prim, ho.t, ho.bary};
         if ((r = shade_jobs(p->devJobs(), p->rayO[cur].as<float4>(), p->rayD[cur].as<float4>(),

@@ -755,15 +755,10 @@ int step_depth(mrb_tracer* t, uint32_t d, StageTimer* tm = nullptr,
     PortionTable pt = portion_table(t);
     // also adds this wavefront to the traced-ray total and clears the next
     // wavefront's counter
-    if ((r = dense_keys(ho.key, cnt + cur, t->maxRays, sc->idBits, t->dense.as<uint32_t>(), pt,
-                        t->stream, t->counters.as<unsigned long long>(), cnt + nxt)))
-        return r;
-    if ((r = radix_sort_pairs<uint32_t>(t->dense.as<uint32_t>(), t->sortedIds.as<uint32_t>(),
-                                        cnt + cur, t->maxRays, 0, 3 + int(sc->idBits), true,
-                                        t->sortTemp.p, t->sortTempBytes, t->stream, true)))
-        return r;
-    if ((r = find_portions(t->dense.as<uint32_t>(), cnt + cur, t->maxRays, sc->idBits, pt,
-                           t->stream)))
+    if ((r = partition_rays(ho.key, cnt + cur, t->maxRays, sc->idBits, t->sortedIds.as<uint32_t>(),
+                            t->dense.as<uint32_t>(), false, pt, t->sortTemp.p, t->sortTempBytes,
+                            t->stream,
+                            t->counters.as<unsigned long long>(), cnt + nxt)))
         return r;
     if (mark(3) || lap(2, 2)) return MRB_E_CUDA;
     HitIn hi{ho.key, ho.prim, ho.t, ho.bary};
@@ -842,14 +837,13 @@ int record_frame(mrb_tracer* t) {
     return step_finalize(t);
 }
 
-// Kernel launches recorded per frame (camera, per depth: trace, dense keys
-// (with the ray count), histogram, histogram scan, onesweep passes
-// (+copy-back), portions, shade; then resolve and frame advance).
+// Kernel launches recorded per frame (camera, per depth: trace, partition
+// (histogram with the ray count, onesweep passes), shade; then resolve and
+// frame advance).
 uint32_t launches_per_frame(const mrb_tracer* t) {
     const uint32_t bits = 3 + t->scene->idBits;
     const uint32_t passes = (bits + 7) / 8;
-    const uint32_t sort = 2 + passes + (passes & 1);
-    uint32_t n = 1 + t->maxDepth * (2 + sort + 2) + 2;
+    uint32_t n = 1 + t->maxDepth * (1 + 1 + passes + 1) + 2;
     if (t->wfpg && t->svoReady) {
         // guiding per guided depth; deposit, leaf averages and the two
         // level filters per frame
@@ -2301,11 +2295,9 @@ int mrb_partition(const uint32_t* keys, uint32_t n, uint32_t idBits, uint32_t* s
     MRB_CUDA(cudaMemcpyAsync(dCount, &n, 4, cudaMemcpyHostToDevice, st));
     PortionTable pt{pOff, pEnd, nonNull};
     int r;
-    if ((r = dense_keys(keys, dCount, n, idBits, sortedDense, pt, st))) return r;
-    if ((r = radix_sort_pairs<uint32_t>(sortedDense, sortedIds, dCount, n, 0, 3 + int(idBits), true,
-                                        sortTmp, sortBytes, st, true)))
+    if ((r = partition_rays(keys, dCount, n, idBits, sortedIds, sortedDense, true, pt, sortTmp,
+                            sortBytes, st)))
         return r;
-    if ((r = find_portions(sortedDense, dCount, n, idBits, pt, st))) return r;
     MRB_CUDA(cudaStreamSynchronize(st));
     return 0;
 }

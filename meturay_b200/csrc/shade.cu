@@ -1,13 +1,8 @@
-// Camera ray generation, ray partitioning helpers, shading and image resolve
+// Camera ray generation, shading and image resolve
 // for the plain wavefront path tracer.
 //
 //   k_camera       KCGenCameraRaysFromArrayGPU + GPUCameraPinhole::GenerateRay
 //                  (GenerationKernels.cuh:26-108, GPUCameraPinhole.cuh:209-243)
-//   k_dense_keys   HitKey -> dense (batch, id) key for the partition sort
-//                  (FillMatIdsForSortKC, RayMemory.cu:17-30)
-//   k_portions     batch boundaries of the sorted keys -> device portion
-//                  table (FindSplitsSparseKC/FindSplitBatchesKC,
-//                  RayMemory.cu:64-104,230-312), found with warp ballots
 //   k_shade        one launch over all non-null rays in partition order:
 //                  PathTracerPathWork / PathTracerBoundaryWork
 //                  (PathTracerKC.cuh:335-649) with Lambert, Metal (GGX) and
@@ -107,57 +102,6 @@ __global__ void __launch_bounds__(256) k_camera(const CameraDev* __restrict__ ca
                                            __uint_as_float(frame));
             chain.nodeB[sid] = make_float4(1.0f, 1.0f, 1.0f, 0.0f);
         }
-    }
-}
-
-// Block 0 also adds the wavefront's ray count to the traced-ray total and
-// clears the next wavefront's counter (where given): two tiny launches less
-// per depth.
-__global__ void __launch_bounds__(256) k_dense_keys(const uint32_t* __restrict__ hitKey,
-                                                    const uint32_t* __restrict__ dCount,
-                                                    uint32_t idBits, uint32_t* __restrict__ dense,
-                                                    PortionTable table,
-                                                    unsigned long long* rayTotal,
-                                                    uint32_t* nextCount) {
-    const uint32_t n = *dCount;
-    if (blockIdx.x == 0 && threadIdx.x < 8) {
-        table.offset[threadIdx.x] = 0;
-        table.end[threadIdx.x] = 0;
-        if (threadIdx.x == 0) {
-            *table.nonNull = n;
-            if (rayTotal) *rayTotal += n;
-            if (nextCount) *nextCount = 0u;
-        }
-    }
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        uint32_t k = hitKey[i];
-        dense[i] = ((k >> kIdBits) << idBits) | (k & ((1u << idBits) - 1u));
-    }
-}
-
-// Batch boundaries of the sorted dense keys.  Each warp compares every key
-// with its predecessor (shuffle, one global read at the warp edge), and the
-// lanes where the batch changes write the portion bounds.
-__global__ void __launch_bounds__(256) k_portions(const uint32_t* __restrict__ sortedDense,
-                                                  const uint32_t* __restrict__ dCount,
-                                                  uint32_t idBits, PortionTable table) {
-    const uint32_t n = *dCount;
-    const uint32_t lane = threadIdx.x & 31;
-    for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += gridDim.x * blockDim.x) {
-        const uint32_t i = base + threadIdx.x;
-        const bool ok = i < n;
-        const uint32_t b = ok ? (sortedDense[i] >> idBits) : 0xFFFFFFFFu;
-        uint32_t prev = __shfl_up_sync(0xFFFFFFFFu, b, 1);
-        uint32_t next = __shfl_down_sync(0xFFFFFFFFu, b, 1);
-        if (lane == 0) prev = (i > 0 && ok) ? (sortedDense[i - 1] >> idBits) : 0xFFFFFFFEu;
-        if (lane == 31) next = (i + 1 < n) ? (sortedDense[i + 1] >> idBits) : 0xFFFFFFFEu;
-        if (!ok) continue;
-        if (i + 1 == n) next = 0xFFFFFFFEu;
-        if (b != prev) {
-            table.offset[b] = i;
-            if (b == kBatchNull) *table.nonNull = i;
-        }
-        if (b != next) table.end[b] = i + 1;
     }
 }
 
@@ -608,23 +552,6 @@ int camera_generate(const CameraDev* cam, const PathOptions& opt, uint32_t baseM
     k_camera<<<grid_for(total, 256, 148 * 16), 256, 0, stream>>>(cam, opt, baseMedium, rayO, rayD,
                                                                 aux, samples, count, total, chain,
                                                                 imgCoords);
-    MRB_CUDA(cudaGetLastError());
-    return 0;
-}
-
-int dense_keys(const uint32_t* hitKey, const uint32_t* dCount, uint32_t maxCount, uint32_t idBits,
-               uint32_t* dense, const PortionTable& table, cudaStream_t stream,
-               unsigned long long* rayTotal, uint32_t* nextCount) {
-    k_dense_keys<<<grid_for(maxCount, 256, 148 * 8), 256, 0, stream>>>(hitKey, dCount, idBits, dense,
-                                                                      table, rayTotal, nextCount);
-    MRB_CUDA(cudaGetLastError());
-    return 0;
-}
-
-int find_portions(const uint32_t* sortedDense, const uint32_t* dCount, uint32_t maxCount,
-                  uint32_t idBits, const PortionTable& table, cudaStream_t stream) {
-    k_portions<<<grid_for(maxCount, 256, 148 * 8), 256, 0, stream>>>(sortedDense, dCount, idBits,
-                                                                    table);
     MRB_CUDA(cudaGetLastError());
     return 0;
 }

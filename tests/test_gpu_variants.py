@@ -1,0 +1,65 @@
+"""Edges of the kernels' variants: tile remainders, the ends of each range that
+a dispatch covers, and the calls on either side of its lines, each against the
+oracle or against the general path of the same library."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _dev(torch, a):
+    return torch.from_numpy(np.ascontiguousarray(a)).cuda()
+
+
+# ---- partition and sort ------------------------------------------------------
+# id bits: the batch bits inside one digit, across two, and at a digit's end
+@pytest.mark.parametrize("id_bits", [1, 5, 6, 7, 8, 13, 14, 24])
+@pytest.mark.parametrize("n", [0, 1, 4095, 4096, 4097, 33000])
+def test_partition_at_digit_and_tile_edges(cuda, oracle, n, id_bits):
+    from meturay_b200._lib import check, lib
+    torch = cuda
+    rng = np.random.default_rng(100 * id_bits + n)
+    batch = rng.choice([0, 1, 2, 4, 6], n).astype(np.uint32)  # some batches absent
+    keys = (batch << 24) | rng.integers(0, 1 << id_bits, n).astype(np.uint32)
+    keys[batch == 0] = 0
+    sid, sd = (torch.full((max(n, 1),), -1, dtype=torch.int32, device="cuda") for _ in range(2))
+    po, pe = (torch.full((8,), 77, dtype=torch.int32, device="cuda") for _ in range(2))
+    nn = torch.full((1,), 77, dtype=torch.int32, device="cuda")
+    tb = lib.mrb_partition_temp_bytes(n, id_bits)
+    tmp = torch.zeros(tb, dtype=torch.uint8, device="cuda")
+    check(lib.mrb_partition(_dev(torch, keys.view(np.int32)).data_ptr() if n else None, n, id_bits,
+                            sid.data_ptr(), sd.data_ptr(), po.data_ptr(), pe.data_ptr(),
+                            nn.data_ptr(), tmp.data_ptr(), tb, None))
+    torch.cuda.synchronize()
+    dense = ((keys >> 24) << id_bits) | (keys & ((1 << id_bits) - 1))
+    order = np.argsort(-dense.astype(np.int64), kind="stable")
+    assert np.array_equal(sid.cpu().numpy()[:n], order)
+    assert np.array_equal(sd.cpu().numpy()[:n].view(np.uint32), dense[order])
+    sorted_batch = batch[order]
+    for b in range(8):
+        at = np.nonzero(sorted_batch == b)[0]
+        want = (at[0], at[-1] + 1) if len(at) else (0, 0)
+        assert (int(po[b]), int(pe[b])) == want, b
+    assert int(nn[0]) == n - int((batch == 0).sum())
+
+
+def test_sort_beyond_the_numbered_flags(cuda):
+    """More pairs than the pass-numbered tile flags hold (2^27): the words are
+    cleared for every pass instead.  Values are the indices, so a stable sort
+    leaves them ascending among equal keys."""
+    from meturay_b200._lib import check, lib
+    torch = cuda
+    n = (1 << 27) + 4097
+    gen = torch.Generator(device="cuda").manual_seed(4)
+    keys = torch.randint(0, 1 << 12, (n,), generator=gen, dtype=torch.int32, device="cuda")
+    vals = torch.arange(n, dtype=torch.int32, device="cuda")
+    orig = keys.clone()
+    tb = lib.mrb_radix_sort_temp_bytes(n, 4, 0, 12)
+    tmp = torch.empty(tb, dtype=torch.uint8, device="cuda")
+    check(lib.mrb_radix_sort_pairs_u32(keys.data_ptr(), vals.data_ptr(), n, 0, 12, 0,
+                                       tmp.data_ptr(), tb, None))
+    torch.cuda.synchronize()
+    assert bool((keys[1:] >= keys[:-1]).all())
+    assert bool(((keys[1:] > keys[:-1]) | (vals[1:] > vals[:-1])).all())
+    assert bool((orig[vals.long()] == keys).all())
+    assert int(vals.long().sum()) == n * (n - 1) // 2
