@@ -1,5 +1,6 @@
-// Learned guiding MLP: the tensor-core forward pass shared by the plain
-// inference kernel (mlp.cu) and the fused guide kernel (learned.cu).
+// Learned guiding MLP: tcgen05 wrappers and operand layouts shared by the
+// inference and training kernels (mlp.cu), and the forward pass of the fused
+// guide kernel (learned.cu), one thread per row.
 //
 // Shared-memory operand layout (no swizzle, "interleaved" core matrices):
 // a core matrix is 8 rows x 16 bytes (8 bf16), its rows 16 bytes apart.
@@ -82,6 +83,11 @@ __device__ __forceinline__ void mbar_init(uint64_t* mbar, uint32_t count) {
                  : "memory");
 }
 
+// The error word may lie in mapped host memory: a plain store.
+__device__ __forceinline__ void set_flag(uint32_t* flag) {
+    *reinterpret_cast<volatile uint32_t*>(flag) = 1u;
+}
+
 // Bounded wait for the phase `parity` of the barrier to complete.
 __device__ __forceinline__ bool mbar_wait(uint64_t* mbar, uint32_t parity) {
     const uint32_t a = smem_u32(mbar);
@@ -124,6 +130,13 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float* v) {
 #pragma unroll
     for (int k = 0; k < 16; k++) v[k] = __uint_as_float(r[k]);
 }
+// One fp32 column of this warp's 32 TMEM lanes.
+__device__ __forceinline__ float tmem_ld1(uint32_t taddr) {
+    uint32_t r;
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];" : "=r"(r) : "r"(taddr));
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+    return __uint_as_float(r);
+}
 __device__ __forceinline__ void tmem_wait_ld() {
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
@@ -164,21 +177,6 @@ __device__ __forceinline__ void store_row(unsigned char* buf, uint32_t row, cons
         *reinterpret_cast<uint4*>(buf + act_offset(row, 8 * c, F)) = q;
     }
 }
-// Read one sample row (F values) of an activation buffer.
-template <int F>
-__device__ __forceinline__ void load_row(const unsigned char* buf, uint32_t row, float* v) {
-#pragma unroll
-    for (int c = 0; c < F / 8; c++) {
-        const uint4 q = *reinterpret_cast<const uint4*>(buf + act_offset(row, 8 * c, F));
-        const uint32_t w[4] = {q.x, q.y, q.z, q.w};
-#pragma unroll
-        for (int k = 0; k < 4; k++) {
-            v[8 * c + 2 * k] = bf16_float(uint16_t(w[k] & 0xFFFFu));
-            v[8 * c + 2 * k + 1] = bf16_float(uint16_t(w[k] >> 16));
-        }
-    }
-}
-
 // Inference keeps no activations for a backward pass: one activation
 // buffer holds the input tile and then each hidden layer in turn (a
 // layer's epilogue overwrites its own operand only after the product has
@@ -198,13 +196,6 @@ static_assert(kMlpTile * kMlpIn * 2 >= kMlpTile * 64 * 2, "x holds a hidden tile
 // TMEM column of the 128 x 64 forward accumulator.
 constexpr uint32_t kColD = 0;
 
-// Bias-gradient accumulators exist only in the training layout.
-template <class SM>
-__device__ __forceinline__ auto clear_dbias(SM& S, int l, int o) -> decltype(S.dbias, void()) {
-    S.dbias[l][o] = 0.0f;
-}
-__device__ __forceinline__ void clear_dbias(MlpFwdSmem&, int, int) {}
-
 // Weights (bf16 image) and biases into shared memory, barrier init, TMEM
 // allocation by warp 0.  Returns the TMEM base address.
 template <class SM>
@@ -215,7 +206,6 @@ __device__ __forceinline__ uint32_t mlp_prologue(SM& S, const MlpDev& m, uint32_
     for (uint32_t i = threadIdx.x; i < kMlpLayers * 64; i += blockDim.x) {
         const int l = int(i / 64), o = int(i % 64);
         S.bias[l][o] = m.params[mlp_layer_offset(l) + (l == 0 ? kMlpIn : 64) * 64 + o];
-        clear_dbias(S, l, o);
     }
     if (threadIdx.x == 0) {
         mbar_init(&S.mbar, 1);
@@ -243,28 +233,6 @@ __device__ __forceinline__ void mlp_epilogue(SM& S, uint32_t tmem, uint32_t cols
     }
 }
 
-// One sample row of the input features into the X buffer (zeros past n).
-template <class SM>
-__device__ __forceinline__ void load_input(SM& S, const float* in, uint32_t n, uint32_t s,
-                                           uint32_t row) {
-    float v[kMlpIn];
-    if (s < n) {
-        const float4* p = reinterpret_cast<const float4*>(in + size_t(s) * kMlpIn);
-#pragma unroll
-        for (int c = 0; c < kMlpIn / 4; c++) {
-            const float4 q = p[c];
-            v[4 * c] = q.x;
-            v[4 * c + 1] = q.y;
-            v[4 * c + 2] = q.z;
-            v[4 * c + 3] = q.w;
-        }
-    } else {
-#pragma unroll
-        for (int c = 0; c < kMlpIn; c++) v[c] = 0.0f;
-    }
-    store_row<kMlpIn>(S.x, row, v);
-}
-
 // Wait for the MMAs committed to S.mbar; on expiry mark the CTA failed.
 // Every thread of the CTA calls it at the same point; the outcome is made
 // common with a block-wide vote so that no thread leaves a barrier behind.
@@ -275,7 +243,7 @@ __device__ __forceinline__ bool mlp_wait(SM& S, uint32_t& phase, uint32_t* error
     ok = __syncthreads_and(ok) != 0;
     if (!ok && threadIdx.x == 0) {
         S.fail = 1;
-        atomicExch(errorFlag, 1u);
+        set_flag(errorFlag);
     }
     tc_fence_after();
     return ok;

@@ -63,3 +63,53 @@ def test_sort_beyond_the_numbered_flags(cuda):
     assert bool(((keys[1:] > keys[:-1]) | (vals[1:] > vals[:-1])).all())
     assert bool((orig[vals.long()] == keys).all())
     assert int(vals.long().sum()) == n * (n - 1) // 2
+
+
+# ---- guiding network ---------------------------------------------------------
+def _network_batch(seed, n):
+    from oracle import mlp as M
+    rng = np.random.default_rng(seed)
+    x = M.encode(rng.uniform(0, 1, (n, 3)), M.sample_sphere(rng, n), M.sample_sphere(rng, n))
+    t = np.zeros((n, 4), np.float32)
+    t[:, :3] = M.sample_sphere(rng, n)
+    t[:, 3] = rng.uniform(0.1, 2.0, n)
+    t[rng.uniform(size=n) < 0.1, 3] = 0.0
+    return x, t
+
+
+# a lone row, the edges of a 128-row tile, and blocks with a second tile
+# (592 inference blocks, 148 training blocks)
+@pytest.mark.parametrize("n", [1, 127, 128, 129, 592 * 128 + 1])
+def test_network_inference_at_tile_edges(system, cuda, n):
+    from meturay_b200.learned import GuideMLP
+    from oracle import mlp as M
+    p = M.init_params(3)
+    x, _ = _network_batch(n, n)
+    out = cuda.full((n + 1, 40), -7.0, dtype=cuda.float32, device="cuda")
+    GuideMLP(system, p).forward(_dev(cuda, x), out)
+    cuda.cuda.synchronize()
+    ref, _ = M.forward(p, x, quantize=True)
+    got = out.cpu().numpy()
+    # as test_gpu_mlp: rounding of the FP32 sums, and a bf16 flip that follows
+    assert np.abs(got[:n] - ref).mean() < 1e-3 * np.abs(ref).mean()
+    assert (got[n] == -7.0).all()  # nothing past the last row
+
+
+@pytest.mark.parametrize("n", [1, 127, 129, 148 * 128 + 1])
+def test_network_gradients_at_tile_edges(system, cuda, n):
+    from meturay_b200.learned import PARAM_COUNT, GuideMLP
+    from oracle import mlp as M
+    p = M.init_params(5)
+    x, t = _network_batch(7 * n, n)
+    t[0, 3] = 1.0
+    grad = cuda.zeros(PARAM_COUNT, dtype=cuda.float32, device="cuda")
+    loss = cuda.zeros(2, dtype=cuda.float32, device="cuda")
+    GuideMLP(system, p).gradients(_dev(cuda, x), _dev(cuda, t), grad, loss)
+    cuda.cuda.synchronize()
+    ref, lsum, wsum = M.gradients(p, x, t, quantize=True)
+    got = grad.cpu().numpy().astype(np.float64)
+    # the bound of test_gpu_mlp's gradients, over the whole vector
+    assert np.linalg.norm(got - ref) < 2e-2 * np.linalg.norm(ref)
+    assert abs(float(loss[0]) - lsum) < 1e-3 * abs(lsum) + 1e-3
+    assert abs(float(loss[1]) - wsum) < 1e-4 * wsum
+    assert (got[M.frozen_mask()] == 0).all()
