@@ -113,3 +113,46 @@ def test_network_gradients_at_tile_edges(system, cuda, n):
     assert abs(float(loss[0]) - lsum) < 1e-3 * abs(lsum) + 1e-3
     assert abs(float(loss[1]) - wsum) < 1e-4 * wsum
     assert (got[M.frozen_mask()] == 0).all()
+
+
+# ---- traversal tree ----------------------------------------------------------
+def _ploc_reference(boxes, radius=16):
+    """Clustering steps and the sum of the inner boxes' half areas, in the same
+    32-bit arithmetic."""
+    c, steps, total = boxes.astype(np.float32), 0, 0.0
+    while len(c) > 1:
+        m = len(c)
+        best, at = np.full(m, np.inf, np.float32), np.where(np.arange(m) == 0, 1, np.arange(m) - 1)
+        for d in [*range(-radius, 0), *range(1, radius + 1)]:
+            i = np.arange(max(0, -d), min(m, m - d))
+            e = np.maximum(c[i, 3:], c[i + d, 3:]) - np.minimum(c[i, :3], c[i + d, :3])
+            a = e[:, 0] * e[:, 1] + e[:, 1] * e[:, 2] + e[:, 2] * e[:, 0]
+            less = a < best[i]
+            best[i[less]], at[i[less]] = a[less], i[less] + d
+        mutual = at[at] == np.arange(m)
+        low, high = mutual & (np.arange(m) < at), mutual & (np.arange(m) > at)
+        j = at[low]
+        c[low] = np.concatenate([np.minimum(c[low, :3], c[j, :3]),
+                                 np.maximum(c[low, 3:], c[j, 3:])], 1)
+        e = c[low, 3:].astype(np.float64) - c[low, :3]
+        total += float((e[:, 0] * e[:, 1] + e[:, 1] * e[:, 2] + e[:, 2] * e[:, 0]).sum())
+        c, steps = c[~high], steps + 1
+    return steps, total
+
+
+# one block's range (1,024 clusters), the first step beyond it, tile remainders
+@pytest.mark.parametrize("n", [2, 3, 33, 1023, 1024, 1025, 1281, 6000])
+def test_ploc_steps_and_areas(system, cuda, n):
+    from meturay_b200 import GPUScene, scenes
+    scene = scenes.random_triangles(n, n)
+    g = GPUScene(system, scene)
+    g.set_wide_tree(1)
+    g.construct_accelerators()
+    a = g.export_accel()
+    steps, area = _ploc_reference(a["tri_aabbs"][a["sorted_idx"]])
+    info = g.accel_info()
+    assert info["ploc_steps"] == steps
+    # the same boxes, summed in double in another order
+    assert abs(info["inner_area_ploc"] - area) <= n * 2.0 ** -52 * area
+    g.construct_accelerators()  # again over the built scene
+    assert g.accel_info()["ploc_steps"] == steps
