@@ -114,15 +114,25 @@ __global__ void k_plan_up(const uint32_t* __restrict__ left, const uint32_t* __r
             const uint32_t j = g - n;
             const uint32_t l = left[j], r = right[j];
             float cl[9], cr[9];
-            for (int k = 1; k <= 8; k++) {
-                cl[k] = (l >= n) ? __ldcg(cost + 8 * size_t(l - n) + (k - 1)) : 0.0f;
-                cr[k] = (r >= n) ? __ldcg(cost + 8 * size_t(r - n) + (k - 1)) : 0.0f;
-            }
+            auto load = [&](uint32_t child, float* c) {
+                float4 a = make_float4(0.0f, 0.0f, 0.0f, 0.0f), b = a;
+                if (child >= n) {
+                    const float4* p = reinterpret_cast<const float4*>(cost + 8 * size_t(child - n));
+                    a = __ldcg(p);
+                    b = __ldcg(p + 1);
+                }
+                c[1] = a.x; c[2] = a.y; c[3] = a.z; c[4] = a.w;
+                c[5] = b.x; c[6] = b.y; c[7] = b.z; c[8] = b.w;
+            };
+            load(l, cl);
+            load(r, cr);
             float E[9];
             uint32_t ks[9];
+#pragma unroll
             for (int c = 2; c <= 8; c++) {
                 float best = 0.0f;
                 uint32_t bk = 0;
+#pragma unroll
                 for (int k = 1; k < c; k++) {
                     const float v = cl[k] + cr[c - k];
                     if (bk == 0 || v < best) {
@@ -140,13 +150,14 @@ __global__ void k_plan_up(const uint32_t* __restrict__ left, const uint32_t* __r
             const float* b = inner + 6 * size_t(j);
             const float dx = b[3] - b[0], dy = b[4] - b[1], dz = b[5] - b[2];
             const float c1 = (dx * dy + dy * dz + dz * dx) + E[8];
-            float* cj = cost + 8 * size_t(j);
             uint32_t single = 0;
-            cj[0] = c1;
             for (int c = 2; c <= 8; c++) {
                 if (c1 <= E[c]) single |= 1u << (c - 1);
-                cj[c - 1] = fminf(c1, E[c]);
+                E[c] = fminf(c1, E[c]);
             }
+            float4* cj = reinterpret_cast<float4*>(cost + 8 * size_t(j));
+            cj[0] = make_float4(c1, E[2], E[3], E[4]);
+            cj[1] = make_float4(E[5], E[6], E[7], E[8]);
             plan[j] = make_uint2(single | (ks[2] << 8) | (ks[3] << 16) | (ks[4] << 24),
                                  ks[5] | (ks[6] << 8) | (ks[7] << 16) | (ks[8] << 24));
             if (g == top) break;
@@ -159,47 +170,14 @@ __device__ __forceinline__ uint32_t plan_byte(uint2 p, int b) {
     return ((b < 4 ? p.x : p.y) >> (8 * (b & 3))) & 0xFFu;
 }
 
-// The children of the wide node made from binary node g under the plan: at
-// most eight, at least two.  Each pending entry holds at least one slot, so
-// at most eight entries are ever pending.
-__device__ __forceinline__ int plan_children(uint32_t g, uint32_t n, const uint32_t* __restrict__ left,
-                                             const uint32_t* __restrict__ right,
-                                             const uint2* __restrict__ plan, uint32_t ch[8]) {
-    uint32_t sg[16];
-    uint8_t si[16], sown[16];
-    int sp = 1, nc = 0;
-    sg[0] = g;
-    si[0] = 8;
-    sown[0] = 1;
-    while (sp > 0) {
-        sp--;
-        const uint32_t x = sg[sp];
-        int i = si[sp];
-        const bool own = sown[sp] != 0;
-        if (!own && (x < n || i == 1)) {
-            ch[nc++] = x;
-            continue;
-        }
-        const uint2 pl = plan[x - n];
-        if (!own && ((pl.x >> (i - 1)) & 1u)) {
-            ch[nc++] = x;
-            continue;
-        }
-        uint32_t k;
-        while ((k = plan_byte(pl, i - 1)) == 0u) i--;
-        // left takes k slots, right i - k (each >= 1)
-        sg[sp] = right[x - n];
-        si[sp] = uint8_t(i - int(k));
-        sown[sp] = 0;
-        sg[sp + 1] = left[x - n];
-        si[sp + 1] = uint8_t(k);
-        sown[sp + 1] = 0;
-        sp += 2;
-    }
-    return nc;
-}
-
-__global__ void __launch_bounds__(128) k_collapse(
+// One level of the collapse: a team of eight lanes makes each wide node of the
+// level's queue, one lane per child slot (four nodes per warp; every lane takes
+// part in the warp's votes and shuffles).  One thread per node spent 68 us on a
+// level however few its nodes (1M triangles, 16 levels): the dependent reads
+// of the plan, the 8 x 8 greedy matching and the eight children's boxes, one
+// after the other.
+constexpr int kCollapseBlock = 128;
+__global__ void __launch_bounds__(kCollapseBlock) k_collapse(
     const WorkItem* __restrict__ qin, const uint32_t* __restrict__ qinCount, WorkItem* qout,
     uint32_t* qoutCount, uint32_t* nodeCounter, uint32_t* triCounter, uint32_t n,
     const uint32_t* __restrict__ left, const uint32_t* __restrict__ right,
@@ -208,168 +186,227 @@ __global__ void __launch_bounds__(128) k_collapse(
     const uint32_t* __restrict__ idx, const uint32_t* __restrict__ key,
     const uint8_t* __restrict__ cull, const uint2* __restrict__ plan, WideNode* nodes, float4* tv0,
     float4* te0, float4* te1) {
+    constexpr uint32_t kAll = 0xFFFFFFFFu;
+    __shared__ uint32_t shNode[kCollapseBlock], shSlots[kCollapseBlock];
+    const uint32_t lane = threadIdx.x & 7u, shift = threadIdx.x & 24u;
+    const uint32_t team0 = threadIdx.x & ~7u;  // the team's first thread
     const uint32_t count = *qinCount;
-    for (uint32_t w = blockIdx.x * blockDim.x + threadIdx.x; w < count;
-         w += gridDim.x * blockDim.x) {
-        const WorkItem it = qin[w];
-        uint32_t ch[8];
-        float area[8];
-        int nc = 2;
-        ch[0] = left[it.bnode - n];
-        ch[1] = right[it.bnode - n];
+    const uint32_t warps = (gridDim.x * kCollapseBlock) >> 5;
+    for (uint32_t w0 = 4u * ((blockIdx.x * kCollapseBlock + threadIdx.x) >> 5); w0 < count;
+         w0 += 4u * warps) {
+        const uint32_t w = w0 + (shift >> 3);
+        const bool valid = w < count;
+        const WorkItem it = valid ? qin[w] : WorkItem{0u, 0u};
+        // ---- children: one per lane, left to right
+        uint32_t x = kInvalid;  // this lane's child
         if (plan) {
-            nc = plan_children(it.bnode, n, left, right, plan, ch);
-        } else {
-            for (int k = 0; k < 2; k++) {
-                float lo[3], hi[3];
-                child_box(ch[k], n, inner, triAabb, sortedIdx, lo, hi);
-                area[k] = (ch[k] >= n) ? half_area(lo, hi) : -1.0f;
+            // lane p with i slots holds p .. p + i - 1; a split keeps the left
+            // child's and hands the right child's to lane p + k
+            uint32_t slots = 0;
+            bool open = false, own = false;
+            if (valid && lane == 0) {
+                x = it.bnode;
+                slots = 8;
+                open = own = true;
             }
-            // open the largest internal child until eight children
-            while (nc < 8) {
-                int best = -1;
-                for (int k = 0; k < nc; k++)
-                    if (ch[k] >= n && (best < 0 || area[k] > area[best])) best = k;
-                if (best < 0) break;
-                const uint32_t b = ch[best];
-                const uint32_t c0 = left[b - n], c1 = right[b - n];
-                ch[best] = c0;
-                ch[nc] = c1;
-                float lo[3], hi[3];
-                child_box(c0, n, inner, triAabb, sortedIdx, lo, hi);
-                area[best] = (c0 >= n) ? half_area(lo, hi) : -1.0f;
-                child_box(c1, n, inner, triAabb, sortedIdx, lo, hi);
-                area[nc] = (c1 >= n) ? half_area(lo, hi) : -1.0f;
-                nc++;
-            }
-        }
-        // slot of each child: the octant of its centroid around the node's
-        // centre, matched greedily by the largest projection on the
-        // octant's diagonal, so that slot ^ (ray octant) orders the
-        // children roughly front to back for any ray direction
-        {
-            float nlo[3], nhi[3];
-            child_box(it.bnode, n, inner, triAabb, sortedIdx, nlo, nhi);
-            float cost[8][8];
-            for (int k = 0; k < nc; k++) {
-                float lo[3], hi[3];
-                child_box(ch[k], n, inner, triAabb, sortedIdx, lo, hi);
-                float dc[3];
-                for (int c = 0; c < 3; c++) dc[c] = (lo[c] + hi[c]) - (nlo[c] + nhi[c]);
-                for (int sl = 0; sl < 8; sl++)
-                    cost[k][sl] = -(((sl & 1) ? dc[0] : -dc[0]) + ((sl & 2) ? dc[1] : -dc[1]) +
-                                    ((sl & 4) ? dc[2] : -dc[2]));
-            }
-            uint32_t slotOf[8];
-            uint32_t usedChild = 0, usedSlot = 0;
-            for (int round = 0; round < nc; round++) {
-                int bk = -1, bs = -1;
-                float bc = 0.0f;
-                for (int k = 0; k < nc; k++) {
-                    if (usedChild & (1u << k)) continue;
-                    for (int sl = 0; sl < 8; sl++) {
-                        if (usedSlot & (1u << sl)) continue;
-                        if (bk < 0 || cost[k][sl] < bc) {
-                            bk = k;
-                            bs = sl;
-                            bc = cost[k][sl];
+            while (__any_sync(kAll, open)) {
+                shSlots[threadIdx.x] = 0;
+                __syncwarp();
+                if (open) {
+                    if (!own && (x < n || slots == 1)) {
+                        open = false;
+                    } else {
+                        const uint2 pl = plan[x - n];
+                        if (!own && ((pl.x >> (slots - 1)) & 1u)) {
+                            open = false;
+                        } else {
+                            uint32_t k;
+                            while ((k = plan_byte(pl, int(slots) - 1)) == 0u) slots--;
+                            // left takes k slots, right the rest (each >= 1)
+                            shNode[threadIdx.x + k] = right[x - n];
+                            shSlots[threadIdx.x + k] = slots - k;
+                            x = left[x - n];
+                            slots = k;
+                            own = false;
                         }
                     }
                 }
-                slotOf[bk] = uint32_t(bs);
-                usedChild |= 1u << bk;
-                usedSlot |= 1u << bs;
+                __syncwarp();
+                if (shSlots[threadIdx.x]) {
+                    x = shNode[threadIdx.x];
+                    slots = shSlots[threadIdx.x];
+                    open = true;
+                }
+                __syncwarp();
             }
-            uint32_t bySlot[8];
-            for (int sl = 0; sl < 8; sl++) bySlot[sl] = kInvalid;
-            for (int k = 0; k < nc; k++) bySlot[slotOf[k]] = ch[k];
-            nc = 8;
-            for (int sl = 0; sl < 8; sl++) ch[sl] = bySlot[sl];
+        } else {
+            // open the largest internal child until eight children
+            float area = -1.0f;  // internal children only
+            auto set = [&](uint32_t g) {
+                x = g;
+                area = -1.0f;
+                if (g >= n) {
+                    float lo[3], hi[3];
+                    child_box(g, n, inner, triAabb, sortedIdx, lo, hi);
+                    area = half_area(lo, hi);
+                    if (!(area == area)) area = 0.0f;  // NaN boxes: any order will do
+                }
+            };
+            if (valid && lane < 2) set(lane == 0 ? left[it.bnode - n] : right[it.bnode - n]);
+            uint32_t nc = 2;
+            while (true) {
+                float best = (x != kInvalid && x >= n) ? area : -1.0f;
+                uint32_t at = lane;
+                bool has = x != kInvalid && x >= n;
+#pragma unroll
+                for (int o = 1; o < 8; o <<= 1) {
+                    const float ob = __shfl_xor_sync(kAll, best, o);
+                    const uint32_t oa = __shfl_xor_sync(kAll, at, o);
+                    const bool oh = __shfl_xor_sync(kAll, has, o);
+                    if (oh && (!has || ob > best || (ob == best && oa < at))) {
+                        best = ob;
+                        at = oa;
+                        has = true;
+                    }
+                }
+                const bool go = valid && has && nc < 8u;
+                if (!__any_sync(kAll, go)) break;
+                const uint32_t b = __shfl_sync(kAll, x, int(at), 8);
+                if (go) {
+                    if (lane == at) set(left[b - n]);
+                    if (lane == nc) set(right[b - n]);
+                    nc++;
+                }
+            }
         }
-        int nInner = 0, nLeaf = 0;
-        for (int k = 0; k < nc; k++)
-            if (ch[k] != kInvalid) (ch[k] >= n) ? nInner++ : nLeaf++;
-        const uint32_t childBase = nInner ? atomicAdd(nodeCounter, uint32_t(nInner)) : 0u;
-        const uint32_t triBase = nLeaf ? atomicAdd(triCounter, uint32_t(nLeaf)) : 0u;
-        const uint32_t qbase = nInner ? atomicAdd(qoutCount, uint32_t(nInner)) : 0u;
+        // ---- slot of each child: the octant of its centroid around the
+        // node's centre, matched greedily by the largest projection on the
+        // octant's diagonal, so that slot ^ (ray octant) orders the children
+        // roughly front to back for any ray direction
+        float blo[3] = {0.0f, 0.0f, 0.0f}, bhi[3] = {0.0f, 0.0f, 0.0f};  // the node's box
+        if (valid) child_box(it.bnode, n, inner, triAabb, sortedIdx, blo, bhi);
+        {
+            float dc[3] = {0.0f, 0.0f, 0.0f};
+            if (x != kInvalid) {
+                float lo[3], hi[3];
+                child_box(x, n, inner, triAabb, sortedIdx, lo, hi);
+                for (int c = 0; c < 3; c++) dc[c] = (lo[c] + hi[c]) - (blo[c] + bhi[c]);
+            }
+            shNode[threadIdx.x] = kInvalid;
+            __syncwarp();
+            uint32_t usedSlot = 0;
+            bool wait = x != kInvalid;  // not placed yet
+            while (__any_sync(kAll, wait)) {
+                float bc = 0.0f;
+                uint32_t bs = 8u, bk = lane;
+#pragma unroll
+                for (uint32_t sl = 0; sl < 8; sl++) {
+                    float cost = -(((sl & 1) ? dc[0] : -dc[0]) + ((sl & 2) ? dc[1] : -dc[1]) +
+                                   ((sl & 4) ? dc[2] : -dc[2]));
+                    if (!(cost == cost)) cost = kFltMax;  // NaN or infinite boxes
+                    if (wait && !((usedSlot >> sl) & 1u) && (bs == 8u || cost < bc)) {
+                        bc = cost;
+                        bs = sl;
+                    }
+                }
+                // least cost, then lowest child, of the team
+#pragma unroll
+                for (int o = 1; o < 8; o <<= 1) {
+                    const float oc = __shfl_xor_sync(kAll, bc, o);
+                    const uint32_t os = __shfl_xor_sync(kAll, bs, o);
+                    const uint32_t ok = __shfl_xor_sync(kAll, bk, o);
+                    if (os != 8u && (bs == 8u || oc < bc || (oc == bc && ok < bk))) {
+                        bc = oc;
+                        bs = os;
+                        bk = ok;
+                    }
+                }
+                if (bs != 8u) {
+                    usedSlot |= 1u << bs;
+                    if (lane == bk) {
+                        shNode[team0 + bs] = x;
+                        wait = false;
+                    }
+                }
+            }
+            __syncwarp();
+            x = shNode[threadIdx.x];  // from here the child in this lane's slot
+            __syncwarp();
+        }
+        const bool isInner = x != kInvalid && x >= n, isLeaf = x != kInvalid && x < n;
+        const uint32_t imask = (__ballot_sync(kAll, isInner) >> shift) & 0xFFu;
+        const uint32_t leafMask = (__ballot_sync(kAll, isLeaf) >> shift) & 0xFFu;
+        uint32_t childBase = 0, triBase = 0, qbase = 0;
+        if (valid && lane == 0) {
+            if (imask) {
+                childBase = atomicAdd(nodeCounter, uint32_t(__popc(imask)));
+                qbase = atomicAdd(qoutCount, uint32_t(__popc(imask)));
+            }
+            if (leafMask) triBase = atomicAdd(triCounter, uint32_t(__popc(leafMask)));
+        }
+        childBase = __shfl_sync(kAll, childBase, 0, 8);
+        triBase = __shfl_sync(kAll, triBase, 0, 8);
+        qbase = __shfl_sync(kAll, qbase, 0, 8);
+        if (!valid) continue;
 
-        // node box = the binary node's box
-        float blo[3], bhi[3];
-        child_box(it.bnode, n, inner, triAabb, sortedIdx, blo, bhi);
+        uint8_t* bytes = reinterpret_cast<uint8_t*>(nodes + it.slot);
         uint32_t e[3];
-        float scale[3];
+        for (int c = 0; c < 3; c++) e[c] = quant_exponent(bhi[c] - blo[c]);
+        if (lane == 0)
+            *reinterpret_cast<float4*>(bytes) = make_float4(
+                blo[0], blo[1], blo[2],
+                __uint_as_float(e[0] | (e[1] << 8) | (e[2] << 16) | (imask << 24)));
+        if (lane == 1)
+            *reinterpret_cast<uint4*>(bytes + 16) = make_uint4(childBase, triBase, leafMask, 0u);
+        float lo[3], hi[3];
+        if (x != kInvalid) child_box(x, n, inner, triAabb, sortedIdx, lo, hi);
         for (int c = 0; c < 3; c++) {
-            e[c] = quant_exponent(bhi[c] - blo[c]);
-            scale[c] = __uint_as_float(e[c] << 23);
-        }
-        uint32_t leafMask = 0;
-        uint8_t q[6][8];
-        for (int c = 0; c < 6; c++)
-            for (int k = 0; k < 8; k++) q[c][k] = (c < 3) ? 255 : 0;  // empty slot never hits
-        uint32_t imask = 0;
-        int ri = 0, rl = 0;
-        for (int k = 0; k < nc; k++) {
-            if (ch[k] == kInvalid) continue;  // empty slot
-            float lo[3], hi[3];
-            child_box(ch[k], n, inner, triAabb, sortedIdx, lo, hi);
-            for (int c = 0; c < 3; c++) {
+            uint32_t q0 = 255u, q1 = 0u;  // an empty slot never hits
+            if (x != kInvalid) {
                 // outward rounding in double: exact for float inputs and
-                // power-of-two scales
-                double ql = floor((double(lo[c]) - double(blo[c])) / double(scale[c]));
-                double qh = ceil((double(hi[c]) - double(blo[c])) / double(scale[c]));
+                // power-of-two scales (the product with 2^(127 - e) is the
+                // quotient)
+                const double inv = __longlong_as_double(int64_t(1150 - int(e[c])) << 52);
+                double ql = floor((double(lo[c]) - double(blo[c])) * inv);
+                double qh = ceil((double(hi[c]) - double(blo[c])) * inv);
                 ql = ql < 0.0 ? 0.0 : (ql > 255.0 ? 255.0 : ql);
                 qh = qh < 0.0 ? 0.0 : (qh > 255.0 ? 255.0 : qh);
-                q[c][k] = static_cast<uint8_t>(ql);
-                q[3 + c][k] = static_cast<uint8_t>(qh);
+                q0 = static_cast<uint32_t>(ql);
+                q1 = static_cast<uint32_t>(qh);
             }
-            if (ch[k] >= n) {
-                imask |= 1u << k;
-                qout[qbase + ri] = WorkItem{ch[k], childBase + uint32_t(ri)};
-                ri++;
-            } else {
-                leafMask |= 1u << k;
-                // leaf: the triangle, reordered into this node's leaf block
-                const uint32_t t = sortedIdx[ch[k]];
-                const uint32_t s = triBase + uint32_t(rl);
-                const uint32_t i0 = idx[3 * size_t(t)], i1 = idx[3 * size_t(t) + 1],
-                               i2 = idx[3 * size_t(t) + 2];
-                const V3 p0 = ld3(pos + 3 * size_t(i0)), p1 = ld3(pos + 3 * size_t(i1)),
-                         p2 = ld3(pos + 3 * size_t(i2));
-                const V3 e0 = p1 - p0, e1 = p2 - p0;
-                tv0[s] = make_float4(p0.x, p0.y, p0.z, __uint_as_float(t));
-                te0[s] = make_float4(e0.x, e0.y, e0.z, __uint_as_float(key[t]));
-                te1[s] = make_float4(e1.x, e1.y, e1.z,
-                                     __uint_as_float(cull ? uint32_t(cull[t]) : 0u));
-                rl++;
-            }
+            bytes[32 + 8 * c + lane] = static_cast<uint8_t>(q0);
+            bytes[56 + 8 * c + lane] = static_cast<uint8_t>(q1);
         }
-        WideNode nd;
-        nd.n0 = make_float4(blo[0], blo[1], blo[2],
-                            __uint_as_float(e[0] | (e[1] << 8) | (e[2] << 16) | (imask << 24)));
-        nd.n1 = make_uint4(childBase, triBase, leafMask, 0u);
-        auto pack = [&](int c, int k0) {
-            return q[c][k0] | (q[c][k0 + 1] << 8) | (q[c][k0 + 2] << 16) |
-                   (uint32_t(q[c][k0 + 3]) << 24);
-        };
-        nd.n2 = make_uint4(pack(0, 0), pack(0, 4), pack(1, 0), pack(1, 4));
-        nd.n3 = make_uint4(pack(2, 0), pack(2, 4), pack(3, 0), pack(3, 4));
-        nd.n4 = make_uint4(pack(4, 0), pack(4, 4), pack(5, 0), pack(5, 4));
-        nodes[it.slot] = nd;
+        const uint32_t below = (1u << lane) - 1u;
+        if (isInner) {
+            const uint32_t r = uint32_t(__popc(imask & below));
+            qout[qbase + r] = WorkItem{x, childBase + r};
+        } else if (isLeaf) {
+            // leaf: the triangle, reordered into this node's leaf block
+            const uint32_t t = sortedIdx[x];
+            const uint32_t s = triBase + uint32_t(__popc(leafMask & below));
+            const uint32_t i0 = idx[3 * size_t(t)], i1 = idx[3 * size_t(t) + 1],
+                           i2 = idx[3 * size_t(t) + 2];
+            const V3 p0 = ld3(pos + 3 * size_t(i0)), p1 = ld3(pos + 3 * size_t(i1)),
+                     p2 = ld3(pos + 3 * size_t(i2));
+            const V3 e0 = p1 - p0, e1 = p2 - p0;
+            tv0[s] = make_float4(p0.x, p0.y, p0.z, __uint_as_float(t));
+            te0[s] = make_float4(e0.x, e0.y, e0.z, __uint_as_float(key[t]));
+            te1[s] = make_float4(e1.x, e1.y, e1.z, __uint_as_float(cull ? uint32_t(cull[t]) : 0u));
+        }
     }
 }
 
+// Counters of a collapse, zeroed before: wide nodes, triangles, then the queue
+// length of each level.
+constexpr int kMaxLevels = 4 * 96;
+constexpr int kCounters = 2 + kMaxLevels + 1;
 __global__ void k_collapse_init(WorkItem* q0, uint32_t* counters, const uint32_t* root) {
     if (threadIdx.x == 0 && blockIdx.x == 0) {
         q0[0] = WorkItem{*root, 0u};
-        counters[0] = 1;  // queue 0 count
-        counters[1] = 0;  // queue 1 count
-        counters[2] = 1;  // node counter (slot 0 = root)
-        counters[3] = 0;  // triangle counter
+        counters[0] = 1;  // slot 0 = root
+        counters[2] = 1;  // level 0
     }
-}
-
-__global__ void k_reset_count(uint32_t* c) {
-    if (threadIdx.x == 0 && blockIdx.x == 0) *c = 0;
 }
 
 // ---------------------------------------------------------------------------
@@ -860,11 +897,13 @@ __global__ void __launch_bounds__(kBlock) k_trace_wide_jobs(const JobDev* __rest
 
 namespace {
 size_t align256(size_t b) { return (b + 255) & ~size_t(255); }
-size_t queue_bytes(uint32_t n) { return align256(size_t(n + 1) * sizeof(WorkItem) * 2 + 64); }
+size_t queue_bytes(uint32_t n) {
+    return align256(size_t(n + 1) * sizeof(WorkItem) * 2 + size_t(kCounters) * 4);
+}
 }  // namespace
 
 size_t wide_scratch_bytes(uint32_t n) {
-    // two work queues of n items + 4 counters; the collapse plan: parents
+    // two work queues of n items and the counters; the collapse plan: parents
     // (2n), arrival flags (n), costs (8n) and plans (n)
     return queue_bytes(n) + align256(size_t(2) * n * 4) + align256(size_t(n) * 4) +
            align256(size_t(8) * n * 4) + align256(size_t(n) * 8);
@@ -898,28 +937,29 @@ int wide_build(const WideBuildIn& in, WideNode* nodes, float4* tv0, float4* te0,
         MRB_CUDA(cudaGetLastError());
         plan = pl;
     }
+    MRB_CUDA(cudaMemsetAsync(counters, 0, size_t(kCounters) * 4, stream));
     k_collapse_init<<<1, 32, 0, stream>>>(q[0], counters, in.root);
     MRB_CUDA(cudaGetLastError());
     // one launch per level; the host checks for an empty queue every 8 levels
-    const uint32_t grid = std::min<uint32_t>((n + 127) / 128, 148u * 8u);
-    for (int level = 0; level < 4 * 96; level++) {
-        const int cur = level & 1;
-        k_reset_count<<<1, 32, 0, stream>>>(counters + (cur ^ 1));
-        k_collapse<<<grid, 128, 0, stream>>>(q[cur], counters + cur, q[cur ^ 1], counters + (cur ^ 1),
-                                             counters + 2, counters + 3, n, in.left, in.right,
-                                             in.inner, in.triAabb, in.sortedIdx, in.pos, in.idx,
-                                             in.key, in.cull, plan, nodes, tv0, te0, te1);
+    const uint32_t grid = std::min<uint32_t>(n / (kCollapseBlock / 8) + 1, 148u * 16u);
+    for (int level = 0; level < kMaxLevels; level++) {
+        uint32_t* qc = counters + 2 + level;
+        k_collapse<<<grid, kCollapseBlock, 0, stream>>>(
+            q[level & 1], qc, q[(level & 1) ^ 1], qc + 1, counters, counters + 1, n, in.left,
+            in.right, in.inner, in.triAabb, in.sortedIdx, in.pos, in.idx, in.key, in.cull, plan,
+            nodes, tv0, te0, te1);
         MRB_CUDA(cudaGetLastError());
         if ((level & 7) == 7) {
-            uint32_t h[4];
-            MRB_CUDA(cudaMemcpyAsync(h, counters, 16, cudaMemcpyDeviceToHost, stream));
+            uint32_t h[2], left = 0;
+            MRB_CUDA(cudaMemcpyAsync(h, counters, 8, cudaMemcpyDeviceToHost, stream));
+            MRB_CUDA(cudaMemcpyAsync(&left, qc + 1, 4, cudaMemcpyDeviceToHost, stream));
             MRB_CUDA(cudaStreamSynchronize(stream));
-            if (h[0] == 0 && h[1] == 0) {
-                if (h[3] != n) {
-                    set_error("wide BVH: %u of %u triangles placed", h[3], n);
+            if (left == 0) {
+                if (h[1] != n) {
+                    set_error("wide BVH: %u of %u triangles placed", h[1], n);
                     return MRB_E_DEVICE;
                 }
-                *nodeCountOut = h[2];
+                *nodeCountOut = h[0];
                 return 0;
             }
         }
