@@ -104,7 +104,7 @@ struct mrb_scene {
     }
     // 8-wide quantised traversal layout, collapsed from the PLOC tree built
     // over the LBVH's sorted leaves (wideTree 1) or from the LBVH itself (0)
-    DBuf wNodes, wTv0, wTe0, wTe1, wScratch;
+    DBuf wNodes, wTv0, wTe0, wTe1;
     uint32_t wNodeCount = 0;
     int traversal = 1;  // 0: binary LBVH nodes, 1: 8-wide nodes
     int wideTree = 2;        // 0 LBVH, 1 PLOC, 2 the one with less inner-box area

@@ -1170,6 +1170,9 @@ int mrb_accel_construct(mrb_scene* s, void* stream) {
         set_error("LBVH: scene has no triangles");
         return MRB_E_ARG;
     }
+    // a rebuild writes over the arrays that frames and hits in flight on any
+    // stream may still read
+    if (s->built) MRB_CUDA(cudaDeviceSynchronize());
     int r = 0;
     const size_t ni = n > 1 ? n - 1 : 1;
     if ((r = s->aTriAabb.alloc(size_t(n) * 24)) || (r = s->aExtent.alloc(32)) ||
@@ -1202,51 +1205,60 @@ int mrb_accel_construct(mrb_scene* s, void* stream) {
         return r;
     if (n >= 2) {
         if ((r = s->wNodes.alloc((n - 1) * sizeof(WideNode))) || (r = s->wTv0.alloc(size_t(n) * 16)) ||
-            (r = s->wTe0.alloc(size_t(n) * 16)) || (r = s->wTe1.alloc(size_t(n) * 16)) ||
-            (r = s->wScratch.alloc(wide_scratch_bytes(n))))
+            (r = s->wTe0.alloc(size_t(n) * 16)) || (r = s->wTe1.alloc(size_t(n) * 16)))
             return r;
+        // everything that lives only through the build comes out of one
+        // allocation: the PLOC tree and its scratch, the collapse's, the probes'
+        auto part = [](size_t bytes) { return (bytes + 255) & ~size_t(255); };
+        const size_t child = part((n - 1) * 4), boxes = part((n - 1) * 24);
+        const size_t collapse = part(std::max(wide_scratch_bytes(n), wide_probe_bytes()));
+        const bool ploc = s->wideTree != 0;
+        DBuf temp;
+        if ((r = temp.alloc(collapse +
+                            (ploc ? 2 * child + boxes + 256 + ploc_scratch_bytes(n) : 0))))
+            return r;
+        char* tp = temp.as<char>() + collapse;
         WideBuildIn wi{n, s->aRoot.as<uint32_t>(), s->aLeft.as<uint32_t>(), s->aRight.as<uint32_t>(),
                        s->aInner.as<float>(), s->aTriAabb.as<float>(), s->aSorted.as<uint32_t>(),
                        s->dPos.as<float>(), s->dIdx.as<uint32_t>(), s->dKey.as<uint32_t>(),
                        s->dCull.as<uint8_t>(), s->wideCollapse};
         // the PLOC tree over the same sorted leaves: tighter upper boxes than
         // the Morton splits give the collapse better nodes to start from
-        DBuf pLeft, pRight, pInner, pRoot, pScratch;
         s->wideTreeUsed = 0;
-        if (s->wideTree != 0) {
-            if ((r = pLeft.alloc((n - 1) * 4)) || (r = pRight.alloc((n - 1) * 4)) ||
-                (r = pInner.alloc((n - 1) * 24)) || (r = pRoot.alloc(4)) ||
-                (r = pScratch.alloc(ploc_scratch_bytes(n))))
-                return r;
+        if (ploc) {
+            uint32_t* pLeft = reinterpret_cast<uint32_t*>(tp);
+            uint32_t* pRight = reinterpret_cast<uint32_t*>(tp + child);
+            float* pInner = reinterpret_cast<float*>(tp + 2 * child);
+            uint32_t* pRoot = reinterpret_cast<uint32_t*>(tp + 2 * child + boxes);
+            void* pScratch = tp + 2 * child + boxes + 256;
             PlocIn pi{n, s->aTriAabb.as<float>(), s->aSorted.as<uint32_t>()};
-            PlocOut po{pLeft.as<uint32_t>(), pRight.as<uint32_t>(), pInner.as<float>(),
-                       pRoot.as<uint32_t>()};
-            if ((r = ploc_build(pi, po, pScratch.p, &s->plocSteps, st))) return r;
-            double* d8 = static_cast<double*>(pScratch.p);
+            PlocOut po{pLeft, pRight, pInner, pRoot};
+            if ((r = ploc_build(pi, po, pScratch, &s->plocSteps, st))) return r;
+            double* d8 = static_cast<double*>(pScratch);
             if ((r = inner_area_sum(s->aInner.as<float>(), n - 1, d8, &s->areaLbvh, st)) ||
-                (r = inner_area_sum(pInner.as<float>(), n - 1, d8, &s->areaPloc, st)))
+                (r = inner_area_sum(pInner, n - 1, d8, &s->areaPloc, st)))
                 return r;
-            pScratch.release();
             if (s->wideTree == 1 || s->areaPloc < s->areaLbvh) {
                 s->wideTreeUsed = 1;
-                wi.root = pRoot.as<uint32_t>();
-                wi.left = pLeft.as<uint32_t>();
-                wi.right = pRight.as<uint32_t>();
-                wi.inner = pInner.as<float>();
+                wi.root = pRoot;
+                wi.left = pLeft;
+                wi.right = pRight;
+                wi.inner = pInner;
             }
         }
         wi.collapse = (s->wideCollapse == kWideCollapseGreedy) ? kWideCollapseGreedy : kWideCollapseSah;
         if ((r = wide_build(wi, s->wNodes.as<WideNode>(), s->wTv0.as<float4>(), s->wTe0.as<float4>(),
-                            s->wTe1.as<float4>(), s->wScratch.p, &s->wNodeCount, st)))
+                            s->wTe1.as<float4>(), temp.p, &s->wNodeCount, st)))
             return r;
         s->wideCollapseUsed = wi.collapse;
         s->collapseProbeBytes[0] = s->collapseProbeBytes[1] = 0.0;
-        s->aNodes2.release();
-        s->aTv02.release();
-        s->aTe02.release();
-        s->aTe12.release();
         s->wAltNodeCount = 0;
-        if (s->wideCollapse == 2) {
+        if (s->wideCollapse != 2) {
+            s->aNodes2.release();
+            s->aTv02.release();
+            s->aTe02.release();
+            s->aTe12.release();
+        } else {
             // both collapses: the layout the probe rays read fewer bytes of is
             // the scene's; the other stays as the alternate that tracers time
             // per depth on their own rays
@@ -1256,11 +1268,12 @@ int mrb_accel_construct(mrb_scene* s, void* stream) {
                 return r;
             wi.collapse = kWideCollapseGreedy;
             if ((r = wide_build(wi, s->aNodes2.as<WideNode>(), s->aTv02.as<float4>(),
-                                s->aTe02.as<float4>(), s->aTe12.as<float4>(), s->wScratch.p,
+                                s->aTe02.as<float4>(), s->aTe12.as<float4>(), temp.p,
                                 &s->wAltNodeCount, st)))
                 return r;
             double pb[2];
-            if ((r = wide_probe_compare(s->wide(), s->wideAlt(), s->aExtent.as<float>(), st, pb)))
+            if ((r = wide_probe_compare(s->wide(), s->wideAlt(), s->aExtent.as<float>(), temp.p, st,
+                                        pb)))
                 return r;
             s->collapseProbeBytes[kWideCollapseSah] = pb[0];
             s->collapseProbeBytes[kWideCollapseGreedy] = pb[1];
@@ -1273,11 +1286,10 @@ int mrb_accel_construct(mrb_scene* s, void* stream) {
                 s->wideCollapseUsed = kWideCollapseGreedy;
             }
         }
-        s->wScratch.release();
         for (float& m : s->wideOrderMs) m = 0.0f;
         if (s->wideOrderMode == MRB_WIDE_AUTO) {
-            if ((r = wide_order_autotune(s->wide(), s->aExtent.as<float>(), st, &s->wideOrder,
-                                         s->wideOrderMs)))
+            if ((r = wide_order_autotune(s->wide(), s->aExtent.as<float>(), temp.p, st,
+                                         &s->wideOrder, s->wideOrderMs)))
                 return r;
         } else {
             s->wideOrder = s->wideOrderMode;
@@ -1422,7 +1434,9 @@ int mrb_accel_set_wide_order(mrb_scene* s, int order) {
     }
     if (!s->built || s->T < 2) return 0;
     if (set_device(s->sys)) return MRB_E_CUDA;
-    return wide_order_autotune(s->wide(), s->aExtent.as<float>(), nullptr, &s->wideOrder,
+    DBuf temp;
+    if (int r = temp.alloc(wide_probe_bytes())) return r;
+    return wide_order_autotune(s->wide(), s->aExtent.as<float>(), temp.p, nullptr, &s->wideOrder,
                                s->wideOrderMs);
 }
 

@@ -1017,41 +1017,62 @@ __global__ void k_probe_rays(const float* __restrict__ ext, uint32_t n, float4* 
 }
 }  // namespace
 
-int wide_order_autotune(const WideAccelDev& acc, const float* dExtent, cudaStream_t st,
-                        int* orderOut, float* msOut) {
-    constexpr uint32_t kProbe = 1u << 16;
-    void* buf = nullptr;
-    const size_t bytes = size_t(kProbe) * (16 + 16 + 4 + 4 + 4 + 8) + 16;
-    MRB_CUDA(cudaMalloc(&buf, bytes));
-    char* b = static_cast<char*>(buf);
-    float4* ro = reinterpret_cast<float4*>(b);
-    float4* rd = ro + kProbe;
-    HitOut ho{reinterpret_cast<uint32_t*>(rd + kProbe), nullptr, nullptr, nullptr};
-    ho.prim = ho.key + kProbe;
-    ho.t = reinterpret_cast<float*>(ho.prim + kProbe);
-    ho.bary = reinterpret_cast<float2*>(ho.t + kProbe);
-    uint32_t* err = reinterpret_cast<uint32_t*>(ho.bary + kProbe);
-    cudaEvent_t e[2];
-    cudaEventCreate(&e[0]);
-    cudaEventCreate(&e[1]);
-    float best[kWideOrders];
-    for (float& b : best) b = 1e30f;
+namespace {
+constexpr uint32_t kProbe = 1u << 16;
+struct ProbeBuffers {
+    float4 *ro, *rd;
+    HitOut ho;
+    unsigned long long* work;  // two pairs of counters
+    uint32_t* err;
+};
+ProbeBuffers probe_buffers(void* scratch) {
+    ProbeBuffers b{};
+    b.ro = static_cast<float4*>(scratch);
+    b.rd = b.ro + kProbe;
+    b.work = reinterpret_cast<unsigned long long*>(b.rd + kProbe);
+    b.ho.bary = reinterpret_cast<float2*>(b.work + 4);
+    b.ho.key = reinterpret_cast<uint32_t*>(b.ho.bary + kProbe);
+    b.ho.prim = b.ho.key + kProbe;
+    b.ho.t = reinterpret_cast<float*>(b.ho.prim + kProbe);
+    b.err = reinterpret_cast<uint32_t*>(b.ho.t + kProbe);
+    return b;
+}
+}  // namespace
+
+size_t wide_probe_bytes() { return size_t(kProbe) * (16 + 16 + 4 + 4 + 4 + 8) + 64; }
+
+int wide_order_autotune(const WideAccelDev& acc, const float* dExtent, void* scratch,
+                        cudaStream_t st, int* orderOut, float* msOut) {
+    const ProbeBuffers b = probe_buffers(scratch);
+    // pass 0, on a few rays, loads the kernels; of the two timed passes the
+    // faster counts.  Everything is enqueued, then waited for once.
+    constexpr int kPasses = 3;
+    cudaEvent_t e[kPasses][kWideOrders + 1] = {};
     int rc = 0;
-    k_probe_rays<<<(kProbe + 255) / 256, 256, 0, st>>>(dExtent, kProbe, ro, rd);
-    for (int rep = 0; rep < 4 && rc == 0; rep++)
-        for (int order = 0; order < kWideOrders && rc == 0; order++) {
-            cudaEventRecord(e[0], st);
-            rc = trace_closest_wide(acc, ro, rd, nullptr, kProbe, ho, err, st, nullptr, order);
-            cudaEventRecord(e[1], st);
-            cudaEventSynchronize(e[1]);
-            float ms = 0.0f;
-            cudaEventElapsedTime(&ms, e[0], e[1]);
-            if (rep > 0) best[order] = std::min(best[order], ms);  // the first pass warms up
+    k_probe_rays<<<(kProbe + 255) / 256, 256, 0, st>>>(dExtent, kProbe, b.ro, b.rd);
+    for (int pass = 0; pass < kPasses && rc == 0; pass++)
+        for (int order = 0; order <= kWideOrders && rc == 0; order++) {
+            if (cudaEventCreate(&e[pass][order]) != cudaSuccess) rc = MRB_E_CUDA;
+            cudaEventRecord(e[pass][order], st);
+            if (rc == 0 && order < kWideOrders)
+                rc = trace_closest_wide(acc, b.ro, b.rd, nullptr, pass ? kProbe : kProbe / 16, b.ho,
+                                        b.err, st, nullptr, order);
         }
-    cudaEventDestroy(e[0]);
-    cudaEventDestroy(e[1]);
-    cudaFree(buf);
+    const cudaError_t waited = cudaStreamSynchronize(st);
+    float best[kWideOrders];
+    for (int o = 0; o < kWideOrders; o++) {
+        best[o] = 1e30f;
+        for (int pass = 1; pass < kPasses && rc == 0; pass++) {
+            float ms = 0.0f;
+            if (cudaEventElapsedTime(&ms, e[pass][o], e[pass][o + 1]) == cudaSuccess)
+                best[o] = std::min(best[o], ms);
+        }
+    }
+    for (auto& pass : e)
+        for (cudaEvent_t ev : pass)
+            if (ev) cudaEventDestroy(ev);
     if (rc) return rc;
+    MRB_CUDA(waited);
     MRB_CUDA(cudaGetLastError());
     int pick = 0;
     for (int o = 1; o < kWideOrders; o++)
@@ -1063,38 +1084,21 @@ int wide_order_autotune(const WideAccelDev& acc, const float* dExtent, cudaStrea
 }
 
 int wide_probe_compare(const WideAccelDev& a, const WideAccelDev& b, const float* dExtent,
-                       cudaStream_t st, double bytesOut[2]) {
-    constexpr uint32_t kProbe = 1u << 16;
-    void* buf = nullptr;
-    const size_t bytes = size_t(kProbe) * (16 + 16 + 4 + 4 + 4 + 8) + 64;
-    MRB_CUDA(cudaMalloc(&buf, bytes));
-    char* base = static_cast<char*>(buf);
-    float4* ro = reinterpret_cast<float4*>(base);
-    float4* rd = ro + kProbe;
-    HitOut ho{reinterpret_cast<uint32_t*>(rd + kProbe), nullptr, nullptr, nullptr};
-    ho.prim = ho.key + kProbe;
-    ho.t = reinterpret_cast<float*>(ho.prim + kProbe);
-    ho.bary = reinterpret_cast<float2*>(ho.t + kProbe);
-    unsigned long long* work = reinterpret_cast<unsigned long long*>(ho.bary + kProbe);
-    uint32_t* err = reinterpret_cast<uint32_t*>(work + 2);
-    int rc = 0;
-    k_probe_rays<<<(kProbe + 255) / 256, 256, 0, st>>>(dExtent, kProbe, ro, rd);
-    for (int which = 0; which < 2 && !rc; which++) {
-        unsigned long long h[2] = {0ull, 0ull};
-        if (cudaMemsetAsync(work, 0, 16 + 4, st) != cudaSuccess) rc = MRB_E_CUDA;
-        if (!rc)
-            rc = trace_closest_wide(which ? b : a, ro, rd, nullptr, kProbe, ho, err, st, work,
-                                    kWideOctant);
-        if (!rc && (cudaMemcpyAsync(h, work, 16, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
-                    cudaStreamSynchronize(st) != cudaSuccess))
-            rc = MRB_E_CUDA;
-        bytesOut[which] = double(h[0]) * double(sizeof(WideNode)) + double(h[1]) * 48.0;
-    }
-    cudaFree(buf);
-    if (rc) {
-        set_error("wide BVH: probe trace failed");
-        return rc;
-    }
+                       void* scratch, cudaStream_t st, double bytesOut[2]) {
+    const ProbeBuffers p = probe_buffers(scratch);
+    MRB_CUDA(cudaMemsetAsync(p.work, 0, 32, st));
+    MRB_CUDA(cudaMemsetAsync(p.err, 0, 4, st));
+    k_probe_rays<<<(kProbe + 255) / 256, 256, 0, st>>>(dExtent, kProbe, p.ro, p.rd);
+    for (int which = 0; which < 2; which++)
+        if (int rc = trace_closest_wide(which ? b : a, p.ro, p.rd, nullptr, kProbe, p.ho, p.err, st,
+                                        p.work + 2 * which, kWideOctant))
+            return rc;
+    unsigned long long h[4] = {0ull, 0ull, 0ull, 0ull};
+    MRB_CUDA(cudaMemcpyAsync(h, p.work, 32, cudaMemcpyDeviceToHost, st));
+    MRB_CUDA(cudaStreamSynchronize(st));
+    for (int which = 0; which < 2; which++)
+        bytesOut[which] = double(h[2 * which]) * double(sizeof(WideNode)) +
+                          double(h[2 * which + 1]) * 48.0;
     return 0;
 }
 
