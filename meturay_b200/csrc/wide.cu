@@ -519,41 +519,33 @@ __device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
     return d;
 }
 
-// The slabs of the octant kernels: plane byte q becomes the float 1 + q / 2^15
-// by one byte permute (bit pattern 0x3F80qq00), so t = q * a + b turns into
-// (1 + q / 2^15) * A + (b - A) with A = 2^15 a: no conversion, and two slots
-// per packed multiply-add.  b - A is rounded once more than b, by at most half
-// an ulp of itself; the near offsets are lowered and the far ones raised by
-// four half ulps (2^-22 of the offset, below 2^-7 of a plane step where A
-// dominates), so a box is never missed that the exact planes would hit.
-// Clusters-1M, camera rays: 1.73 ms with the plane bytes converted one by one
-// (near planes by a permute to 2^23 + q and a subtraction, far planes on the
-// XU pipe), 1.61 ms so; 2^15 and not 2^23 because the margin shrinks with the
-// scale: at 2^23 it is 1.5 plane steps and the extra visits cost more.  The
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+    uint64_t d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+
+// The slabs of the octant kernels, two slots per packed instruction.  The bytes
+// of the near planes become floats by a permute under the exponent of 2^23 and
+// one addition that takes 2^23 off again, those of the far planes on the XU pipe,
+// and one multiply-add gives two planes, bit for bit the values of child_span.
+// The node loop is bound by instructions issued.  Clusters 1M, camera rays: 1.75
+// ms with one slot per instruction, 1.60 ms so, 1.63 ms with the far planes by
+// permutes too; a million incoherent rays (refill) 1.00, 0.94 and 0.97 ms.  The
 // sorted kernels keep the plain form, which is no slower there.
 struct PackedSlabs {
-    uint64_t ax, ay, az;     // (A, A)
-    uint64_t nx, ny, nz;     // near offsets, twice
-    uint64_t fx, fy, fz;     // far offsets
+    uint64_t ax, ay, az, bx, by, bz;  // each twice
 };
 __device__ __forceinline__ PackedSlabs packed_slabs(const NodeSlabs& s) {
-    PackedSlabs p;
-    auto axis = [](float a, float b, uint64_t& A, uint64_t& n, uint64_t& f) {
-        const float k = a * 32768.0f, c = b - k;
-        const float lo = __fmaf_rn(fabsf(c), -0x1p-22f, c), hi = __fmaf_rn(fabsf(c), 0x1p-22f, c);
-        A = pack2(k, k);
-        n = pack2(lo, lo);
-        f = pack2(hi, hi);
-    };
-    axis(s.ax, s.bx, p.ax, p.nx, p.fx);
-    axis(s.ay, s.by, p.ay, p.ny, p.fy);
-    axis(s.az, s.bz, p.az, p.nz, p.fz);
-    return p;
+    return {pack2(s.ax, s.ax), pack2(s.ay, s.ay), pack2(s.az, s.az),
+            pack2(s.bx, s.bx), pack2(s.by, s.by), pack2(s.bz, s.bz)};
 }
-template <int kk>
+template <int kk, bool kXu>
 __device__ __forceinline__ uint64_t plane_pair(uint32_t w) {
-    return pack2(__uint_as_float(__byte_perm(w, 0x3F800000u, 0x7604u | (kk << 4))),
-                 __uint_as_float(__byte_perm(w, 0x3F800000u, 0x7604u | ((kk + 1) << 4))));
+    if constexpr (kXu) return pack2(float(byte_of(w, kk)), float(byte_of(w, kk + 1)));
+    return add2(pack2(__uint_as_float(__byte_perm(w, 0x4B000000u, 0x7550u | kk)),
+                      __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7550u | (kk + 1)))),
+                pack2(-8388608.0f, -8388608.0f));
 }
 // Entry and exit distances of child slots k and k + 1 (compile-time, k even).
 template <int k>
@@ -561,12 +553,12 @@ __device__ __forceinline__ void child_spans(const NodeSlabs& s, const PackedSlab
                                             float closest, float tn[2], float tf[2]) {
     constexpr int h = k < 4 ? 0 : 1, kk = k & 3;
     float nx[2], ny[2], nz[2], fx[2], fy[2], fz[2];
-    unpack2(fma2(plane_pair<kk>(s.qn[0 + h]), p.ax, p.nx), nx[0], nx[1]);
-    unpack2(fma2(plane_pair<kk>(s.qn[2 + h]), p.ay, p.ny), ny[0], ny[1]);
-    unpack2(fma2(plane_pair<kk>(s.qn[4 + h]), p.az, p.nz), nz[0], nz[1]);
-    unpack2(fma2(plane_pair<kk>(s.qf[0 + h]), p.ax, p.fx), fx[0], fx[1]);
-    unpack2(fma2(plane_pair<kk>(s.qf[2 + h]), p.ay, p.fy), fy[0], fy[1]);
-    unpack2(fma2(plane_pair<kk>(s.qf[4 + h]), p.az, p.fz), fz[0], fz[1]);
+    unpack2(fma2(plane_pair<kk, false>(s.qn[0 + h]), p.ax, p.bx), nx[0], nx[1]);
+    unpack2(fma2(plane_pair<kk, false>(s.qn[2 + h]), p.ay, p.by), ny[0], ny[1]);
+    unpack2(fma2(plane_pair<kk, false>(s.qn[4 + h]), p.az, p.bz), nz[0], nz[1]);
+    unpack2(fma2(plane_pair<kk, true>(s.qf[0 + h]), p.ax, p.bx), fx[0], fx[1]);
+    unpack2(fma2(plane_pair<kk, true>(s.qf[2 + h]), p.ay, p.by), fy[0], fy[1]);
+    unpack2(fma2(plane_pair<kk, true>(s.qf[4 + h]), p.az, p.bz), fz[0], fz[1]);
 #pragma unroll
     for (int j = 0; j < 2; j++) {
         tn[j] = fmaxf(fmaxf(nx[j], ny[j]), fmaxf(nz[j], tmin));
