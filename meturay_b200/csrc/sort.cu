@@ -42,6 +42,26 @@ constexpr int kThreads = 256;
 constexpr int kWarps = kThreads / 32;
 constexpr int kItems = 16;
 constexpr int kTile = kThreads * kItems;  // 4096
+// Up to kSmallCount elements the tiles are of 1,024, up to kMidCount of 2,048:
+// the block's serial part (the ranking, item by item) is shorter and more SMs
+// work, while the look-back has more tiles to walk.  Three passes of 32-bit pairs
+// with kTile and with these tiles: 65,536 pairs 65 and 43 us, 300,000 73 and 57,
+// 600,000 80 and 67; at 1,000,000 both take 99.
+constexpr int kSmallItems = 4, kMidItems = 8;
+constexpr uint32_t kSmallCount = 200u * kThreads * kSmallItems;
+constexpr uint32_t kMidCount = 320u * kThreads * kMidItems;
+__host__ __device__ __forceinline__ uint32_t tile_size(uint32_t n) {
+    return uint32_t(kThreads) * (n <= kSmallCount ? kSmallItems : n <= kMidCount ? kMidItems : kItems);
+}
+__host__ __device__ __forceinline__ uint32_t tile_count(uint32_t n) {
+    const uint32_t t = tile_size(n);
+    return n / t + (n % t ? 1u : 0u);
+}
+// Most tiles of any count up to maxCount.
+inline uint32_t max_tiles(uint32_t maxCount) {
+    return std::max({tile_count(maxCount), tile_count(std::min(maxCount, kMidCount)),
+                     tile_count(std::min(maxCount, kSmallCount))});
+}
 constexpr uint32_t kSpinLimit = 1u << 24;
 constexpr int kLook = 8;  // predecessors read at once by the look-back
 
@@ -100,7 +120,7 @@ __global__ void __launch_bounds__(kThreads) k_histogram(const K* __restrict__ ke
     const uint32_t n = dCount ? *dCount : hCount;
     const uint32_t first = blockIdx.x * kThreads + threadIdx.x, stride = gridDim.x * kThreads;
     if (clearStatus) {
-        const uint32_t words = (n / kTile + (n % kTile ? 1u : 0u)) * 256u;
+        const uint32_t words = tile_count(n) * 256u;
         for (uint32_t i = first; i < words; i += stride) status[i] = 0u;
     }
     if (kDense && blockIdx.x == 0 && threadIdx.x < 8) {
@@ -182,27 +202,44 @@ __device__ __forceinline__ void block_exclusive2(uint32_t a, uint32_t b, uint32_
 // and the values are read when they are needed, at 128 registers two blocks ran.
 template <class K>
 constexpr int kSweepBlocks = sizeof(K) == 8 ? 3 : 4;
-template <class K, bool kDense>
-__global__ void __launch_bounds__(kThreads, kSweepBlocks<K>) k_onesweep(
-    const K* __restrict__ keysIn, K* __restrict__ keysOut, const uint32_t* __restrict__ valsIn,
-    uint32_t* __restrict__ valsOut, const uint32_t* __restrict__ dCount, uint32_t hCount,
+// Lanes of vmask with this lane's digit.  A match takes a turn per distinct
+// digit, a vote per bit eight turns always.  The 64-bit keys are Morton codes,
+// whose low digits are random: 1M pairs, eight passes, 244 us with matches and 214
+// with votes.  The 32-bit keys have few distinct digits in a warp in most sorts:
+// 8M pairs of 37 different keys 342 us with matches and 472 with votes.
+template <class K>
+__device__ __forceinline__ uint32_t same_digit(uint32_t vmask, uint32_t dig) {
+    if constexpr (sizeof(K) == 4) return __match_any_sync(vmask, dig);
+    uint32_t peers = vmask;
+#pragma unroll
+    for (int b = 0; b < 8; b++) {
+        const bool on = (dig >> b) & 1u;
+        const uint32_t v = __ballot_sync(vmask, on);
+        peers &= on ? v : ~v;
+    }
+    return peers;
+}
+
+template <class K, bool kDense, int kN>
+__device__ __forceinline__ void sweep_tiles(
+    SortSmem<K>& sm, const K* __restrict__ keysIn, K* __restrict__ keysOut,
+    const uint32_t* __restrict__ valsIn, uint32_t* __restrict__ valsOut, uint32_t n,
     const uint32_t* __restrict__ hist, uint32_t* tileStatus, uint32_t* tileTicket, int bit,
-    int nbits, int desc, StatusFlags flags, PartitionJob P, uint32_t* errorFlag) {
-    extern __shared__ __align__(16) unsigned char smemRaw[];
-    SortSmem<K>& sm = *reinterpret_cast<SortSmem<K>*>(smemRaw);
+    int nbits, int desc, const StatusFlags& flags, const PartitionJob& P, uint32_t* errorFlag) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint32_t mask = (1u << nbits) - 1u;
     const uint32_t ltMask = (1u << lane) - 1u;
-    const uint32_t n = dCount ? *dCount : hCount;
-    const uint32_t tiles = n / kTile + (n % kTile ? 1u : 0u);
-
+    const uint32_t tiles = tile_count(n);
+    // more blocks than tiles would crowd the tiles on the SMs that start first
+    // (480 blocks for 245 tiles of a million pairs: 128 us, 99 us so)
+    if (blockIdx.x >= tiles) return;
     for (;;) {
         if (tid == 0) sm.tile = atomicAdd(tileTicket, 1u);
         __syncthreads();
         const uint32_t tile = sm.tile;
         if (tile >= tiles) return;
         for (int i = tid; i < kWarps * 256; i += kThreads) (&sm.warpHist[0][0])[i] = 0;
-        const uint32_t base = tile * kTile;
+        const uint32_t base = tile * uint32_t(kThreads * kN);
         if (kDense && tile == 0) {
             // portions of the descending order: a batch follows all higher ones
             if (tid < 8) sm.batch[tid] = batch_straddles(P.idBits) ? P.batchCount[tid] : 0u;
@@ -227,12 +264,12 @@ __global__ void __launch_bounds__(kThreads, kSweepBlocks<K>) k_onesweep(
         }
         __syncthreads();
 
-        // ---- load: warp w owns [base + w*512, base + (w+1)*512), item-major ----
-        K key[kItems];
-        uint32_t place[kItems];  // digit << 16 | rank
-        const uint32_t wbase = base + warp * (32 * kItems);
+        // ---- load: warp w owns 32 * kN elements, item-major ----
+        K key[kN];
+        uint32_t place[kN];  // digit << 16 | rank
+        const uint32_t wbase = base + warp * (32 * kN);
 #pragma unroll
-        for (int i = 0; i < kItems; i++) {
+        for (int i = 0; i < kN; i++) {
             uint32_t idx = wbase + i * 32 + lane;
             bool ok = idx < n;
             key[i] = ok ? read_key<kDense>(keysIn[idx], P.idBits) : K(0);
@@ -240,13 +277,13 @@ __global__ void __launch_bounds__(kThreads, kSweepBlocks<K>) k_onesweep(
         // ---- warp-level multisplit ranking (stable: item-major, lane order) ----
         uint32_t* wh = sm.warpHist[warp];
 #pragma unroll
-        for (int i = 0; i < kItems; i++) {
+        for (int i = 0; i < kN; i++) {
             uint32_t idx = wbase + i * 32 + lane;
             bool ok = idx < n;
             uint32_t vmask = __ballot_sync(0xFFFFFFFFu, ok);
             if (ok) {
                 const uint32_t dig = digit_of(key[i], bit, mask, desc != 0);
-                uint32_t peers = __match_any_sync(vmask, dig);
+                const uint32_t peers = same_digit<K>(vmask, dig);
                 uint32_t prior = wh[dig];
                 __syncwarp(vmask);
                 if (lane == (__ffs(peers) - 1)) wh[dig] = prior + __popc(peers);
@@ -256,6 +293,16 @@ __global__ void __launch_bounds__(kThreads, kSweepBlocks<K>) k_onesweep(
         }
         __syncthreads();
 
+        // the values: in flight during the look-back where registers are left
+        constexpr bool kEarly = kN <= kMidItems;
+        uint32_t val[kEarly ? kN : 1];
+        if constexpr (kEarly) {
+#pragma unroll
+            for (int i = 0; i < kN; i++) {
+                const uint32_t idx = wbase + i * 32 + lane;
+                val[i] = valsIn ? (idx < n ? valsIn[idx] : 0u) : idx;
+            }
+        }
         // ---- per digit: warp prefix, tile count, look-back ----
         {
             const uint32_t d = tid;  // kThreads == 256 digits
@@ -311,13 +358,14 @@ __global__ void __launch_bounds__(kThreads, kSweepBlocks<K>) k_onesweep(
 
         // ---- reorder the tile through shared memory ----
 #pragma unroll
-        for (int i = 0; i < kItems; i++) {
+        for (int i = 0; i < kN; i++) {
             uint32_t idx = wbase + i * 32 + lane;
             if (idx < n) {
                 const uint32_t dig = place[i] >> 16;
                 uint32_t p = sm.digitStart[dig] + sm.warpHist[warp][dig] + (place[i] & 0xFFFFu);
                 sm.keys[p] = key[i];
-                sm.vals[p] = valsIn ? valsIn[idx] : idx;
+                if constexpr (kEarly) sm.vals[p] = val[i];
+                else sm.vals[p] = valsIn ? valsIn[idx] : idx;
             }
         }
         __syncthreads();
@@ -331,6 +379,28 @@ __global__ void __launch_bounds__(kThreads, kSweepBlocks<K>) k_onesweep(
         }
         __syncthreads();
     }
+}
+
+template <class K, bool kDense>
+__global__ void __launch_bounds__(kThreads, kSweepBlocks<K>) k_onesweep(
+    const K* __restrict__ keysIn, K* __restrict__ keysOut, const uint32_t* __restrict__ valsIn,
+    uint32_t* __restrict__ valsOut, const uint32_t* __restrict__ dCount, uint32_t hCount,
+    const uint32_t* __restrict__ hist, uint32_t* tileStatus, uint32_t* tileTicket, int bit,
+    int nbits, int desc, StatusFlags flags, PartitionJob P, uint32_t* errorFlag) {
+    extern __shared__ __align__(16) unsigned char smemRaw[];
+    SortSmem<K>& sm = *reinterpret_cast<SortSmem<K>*>(smemRaw);
+    const uint32_t n = dCount ? *dCount : hCount;
+    if (n <= kSmallCount)
+        sweep_tiles<K, kDense, kSmallItems>(sm, keysIn, keysOut, valsIn, valsOut, n, hist,
+                                            tileStatus, tileTicket, bit, nbits, desc, flags, P,
+                                            errorFlag);
+    else if (n <= kMidCount)
+        sweep_tiles<K, kDense, kMidItems>(sm, keysIn, keysOut, valsIn, valsOut, n, hist,
+                                          tileStatus, tileTicket, bit, nbits, desc, flags, P,
+                                          errorFlag);
+    else
+        sweep_tiles<K, kDense, kItems>(sm, keysIn, keysOut, valsIn, valsOut, n, hist, tileStatus,
+                                       tileTicket, bit, nbits, desc, flags, P, errorFlag);
 }
 
 template <class K>
@@ -387,7 +457,7 @@ int sort_impl(const K* srcKeys, const uint32_t* srcVals, K* dstKeys, uint32_t* d
         return -1;
     }
     const int passes = (endBit - beginBit + 7) / 8;
-    const uint32_t tiles = maxCount / kTile + (maxCount % kTile ? 1u : 0u);
+    const uint32_t tiles = max_tiles(maxCount);
     unsigned char* p = static_cast<unsigned char*>(temp);
     uint32_t* hist = reinterpret_cast<uint32_t*>(p);
     uint32_t* tickets = hist + 8 * 256;
@@ -444,7 +514,7 @@ int sort_impl(const K* srcKeys, const uint32_t* srcVals, K* dstKeys, uint32_t* d
 
 size_t radix_sort_temp_bytes(uint32_t maxCount, int keyBytes, int beginBit, int endBit) {
     const int passes = (endBit - beginBit + 7) / 8;
-    const size_t tiles = (size_t(maxCount) + kTile - 1) / kTile;
+    const size_t tiles = max_tiles(maxCount);
     size_t bytes = 0;
     bytes += align_up(kHeadBytes);                          // histograms, tickets, error flag
     bytes += align_up((tiles + 1) * 256 * 4);               // tile status

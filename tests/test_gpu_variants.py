@@ -43,22 +43,37 @@ def test_partition_at_digit_and_tile_edges(cuda, oracle, n, id_bits):
     assert int(nn[0]) == n - int((batch == 0).sum())
 
 
+def _sorted_on_device(torch, n, bits, seed):
+    from meturay_b200._lib import check, lib
+    gen = torch.Generator(device="cuda").manual_seed(seed)
+    keys = torch.randint(0, 1 << bits, (n,), generator=gen, dtype=torch.int32, device="cuda")
+    vals = torch.arange(n, dtype=torch.int32, device="cuda")
+    orig = keys.clone()
+    tb = lib.mrb_radix_sort_temp_bytes(n, 4, 0, bits)
+    tmp = torch.empty(tb, dtype=torch.uint8, device="cuda")
+    check(lib.mrb_radix_sort_pairs_u32(keys.data_ptr(), vals.data_ptr(), n, 0, bits, 0,
+                                       tmp.data_ptr(), tb, None))
+    torch.cuda.synchronize()
+    return orig, keys, vals
+
+
+# the lines between tiles of 1,024, 2,048 and 4,096 elements
+@pytest.mark.parametrize("n", [1, 1024, 1025, 204_800, 204_801, 655_360, 655_361])
+def test_sort_at_tile_size_lines(cuda, n):
+    torch = cuda
+    orig, keys, vals = _sorted_on_device(torch, n, 20, n)
+    want, order = torch.sort(orig, stable=True)
+    assert torch.equal(keys, want)
+    assert torch.equal(vals.long(), order)
+
+
 def test_sort_beyond_the_numbered_flags(cuda):
     """More pairs than the pass-numbered tile flags hold (2^27): the words are
     cleared for every pass instead.  Values are the indices, so a stable sort
     leaves them ascending among equal keys."""
-    from meturay_b200._lib import check, lib
     torch = cuda
     n = (1 << 27) + 4097
-    gen = torch.Generator(device="cuda").manual_seed(4)
-    keys = torch.randint(0, 1 << 12, (n,), generator=gen, dtype=torch.int32, device="cuda")
-    vals = torch.arange(n, dtype=torch.int32, device="cuda")
-    orig = keys.clone()
-    tb = lib.mrb_radix_sort_temp_bytes(n, 4, 0, 12)
-    tmp = torch.empty(tb, dtype=torch.uint8, device="cuda")
-    check(lib.mrb_radix_sort_pairs_u32(keys.data_ptr(), vals.data_ptr(), n, 0, 12, 0,
-                                       tmp.data_ptr(), tb, None))
-    torch.cuda.synchronize()
+    orig, keys, vals = _sorted_on_device(torch, n, 12, 4)
     assert bool((keys[1:] >= keys[:-1]).all())
     assert bool(((keys[1:] > keys[:-1]) | (vals[1:] > vals[:-1])).all())
     assert bool((orig[vals.long()] == keys).all())
