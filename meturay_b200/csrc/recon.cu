@@ -260,22 +260,33 @@ __global__ void __launch_bounds__(256) k_filter_grid_tiled(const float4* __restr
     const int32_t tx0 = (static_cast<int32_t>(blockIdx.x) % tilesX) * kFilterTile;
     const int32_t ty0 = (static_cast<int32_t>(blockIdx.x) / tilesX) * kFilterTile;
     const int32_t ox = (tx0 - hi) * S, oy = (ty0 - hi) * S;      // staged origin (samples)
+    // A sample's coordinates may round into the pixel beside its own.  Where
+    // no staged sample's did (nearly every tile), the windows need not be
+    // widened by that pixel: with one sample per pixel and a 3-pixel window, 9
+    // candidates per pixel instead of 25 (1080p, the same window: 107 -> 75 us with
+    // one sample per pixel, 355 -> 238 us with four).
+    bool own = true;
     for (int32_t i = threadIdx.x; i < span * span; i += blockDim.x) {
         const int32_t ly = i / span, lx = i - ly * span;
         const int32_t sy = oy + ly, sx = ox + lx;
         if (sy >= 0 && sy < SH && sx >= 0 && sx < SW) {
             const size_t sid = size_t(sy) * size_t(SW) + size_t(sx);
-            sc[i] = coords[sid];
+            const float2 c = coords[sid];
+            sc[i] = c;
             sv[i] = samples[sid];
+            const SamplePix s = sample_pix(c.x, c.y, f.wh);
+            own = own && s.ok && s.ix == sx / S && s.iy == sy / S;
         }
     }
-    __syncthreads();
+    const int32_t slack = __syncthreads_and(own) ? 0 : 1;
     const int32_t px = tx0 + static_cast<int32_t>(threadIdx.x) % kFilterTile;
     const int32_t py = ty0 + static_cast<int32_t>(threadIdx.x) / kFilterTile;
     if (px >= static_cast<int32_t>(width) || py >= static_cast<int32_t>(height)) return;
     const float pcx = static_cast<float>(px) + 0.5f, pcy = static_cast<float>(py) + 0.5f;
-    const int32_t sy0 = max(0, (py - hi) * S), sy1 = min(SH, (py - loMin + 2) * S);
-    const int32_t sx0 = max(0, (px - hi) * S), sx1 = min(SW, (px - loMin + 2) * S);
+    const int32_t sy0 = max(0, (py - hi + 1 - slack) * S),
+                  sy1 = min(SH, (py - loMin + 1 + slack) * S);
+    const int32_t sx0 = max(0, (px - hi + 1 - slack) * S),
+                  sx1 = min(SW, (px - loMin + 1 + slack) * S);
     float ax = 0.0f, ay = 0.0f, az = 0.0f, wsum = 0.0f;
     for (int32_t sy = sy0; sy < sy1; sy++)
         for (int32_t sx = sx0; sx < sx1; sx++) {
