@@ -4,12 +4,14 @@
 // expands every sample to the pixels its filter reaches (one (pixel,
 // sample) pair per pixel), radix-sorts the pairs by pixel and reduces each
 // pixel's run with a block or warp reduction.  Here:
-//   - the general entry point (any image coordinates) keeps that structure,
-//     but compacts the valid pairs first (count, scan, write in sample
-//     order), sorts only those with the onesweep sort on the pixel bits,
-//     keeps the element count on the device (no host round trip, so the
-//     splat can sit inside a captured graph) and sums each pixel's run in
-//     one thread in ascending sample order;
+//   - the general entry point (any image coordinates) sorts a list with the
+//     onesweep sort, its length staying on the device (no host round trip, so
+//     the splat can sit inside a captured graph), and every pixel sums its
+//     samples in ascending sample order.  With a window of one or two pixels
+//     the list holds the pairs of pixel and sample (count, scan, write in sample
+//     order) and a thread sums a pixel's run; with larger ones it holds a
+//     sample once per tile of 8 x 8 pixels that its window touches, and a warp
+//     walks a tile's samples for half of its pixels;
 //   - the tracer's own samples lie on the camera's stratified grid, so each
 //     pixel finds its candidates by index arithmetic in a small
 //     neighbourhood and sums them in the same ascending sample order: the
@@ -18,6 +20,7 @@
 // own CPU expectation (Test_TracerCUDA/T_ReconFilter.cu:96-140).
 #include <cmath>
 #include <cstring>
+#include <type_traits>
 #include <vector>
 
 #include "../../include/mrb200.h"
@@ -77,6 +80,9 @@ __host__ __device__ inline bool in_segment(const ImageSeg& g, int32_t px, int32_
            px < g.offX + g.w && py >= g.offY && py < g.offY + g.h;
 }
 
+// ---------------------------------------------------------------------------
+// Windows of one or two pixels: pairs of pixel and sample
+// ---------------------------------------------------------------------------
 // Pass 1: number of (pixel, sample) pairs per sample.
 __global__ void __launch_bounds__(256) k_expand_count(const float2* __restrict__ coords, uint32_t n,
                                                       ReconFilterDev f, ImageSeg g,
@@ -184,6 +190,175 @@ __global__ void __launch_bounds__(256) k_filter_pixels(
         }
         counts[q] += wsum;
     }
+}
+
+// ---------------------------------------------------------------------------
+// Larger windows: tiles of pixels
+// ---------------------------------------------------------------------------
+// Tiles of the segment that a sample's window touches.
+constexpr int32_t kTileSide = 8;
+struct TileSpan {
+    int32_t x0, x1, y0, y1;  // [x0, x1) x [y0, y1)
+};
+__device__ __forceinline__ TileSpan tile_span(const SamplePix& s, const ImageSeg& g) {
+    if (!s.ok) return {0, 0, 0, 0};
+    // the window, relative to the segment and clipped to its pixels in the image
+    const int64_t x = int64_t(s.ix) - g.offX, y = int64_t(s.iy) - g.offY;
+    const int64_t ax = max(x + s.x0, int64_t(max(0, -g.offX)));
+    const int64_t bx = min(x + s.x1, int64_t(min(g.w, g.resW - g.offX)));
+    const int64_t ay = max(y + s.y0, int64_t(max(0, -g.offY)));
+    const int64_t by = min(y + s.y1, int64_t(min(g.h, g.resH - g.offY)));
+    if (ax >= bx || ay >= by) return {0, 0, 0, 0};
+    return {int32_t(ax) / kTileSide, int32_t(bx - 1) / kTileSide + 1,
+            int32_t(ay) / kTileSide, int32_t(by - 1) / kTileSide + 1};
+}
+
+// Pass 1: number of tiles per sample.
+__global__ void __launch_bounds__(256) k_tile_count(const float2* __restrict__ coords, uint32_t n,
+                                                    uint32_t wh, ImageSeg g,
+                                                    uint32_t* __restrict__ count) {
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const float2 c = coords[i];
+        const TileSpan t = tile_span(sample_pix(c.x, c.y, wh), g);
+        count[i] = uint32_t(t.x1 - t.x0) * uint32_t(t.y1 - t.y0);
+    }
+}
+
+// Pass 2: the (tile, sample) entries, at the sample's scanned offset.
+__global__ void __launch_bounds__(256) k_tile_write(const float2* __restrict__ coords, uint32_t n,
+                                                    uint32_t wh, ImageSeg g, int32_t tilesX,
+                                                    const uint32_t* __restrict__ offset,
+                                                    uint32_t* __restrict__ keys,
+                                                    uint32_t* __restrict__ vals) {
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const float2 c = coords[i];
+        const TileSpan t = tile_span(sample_pix(c.x, c.y, wh), g);
+        uint32_t o = offset[i];
+        for (int32_t y = t.y0; y < t.y1; y++)
+            for (int32_t x = t.x0; x < t.x1; x++) {
+                keys[o] = static_cast<uint32_t>(y * tilesX + x);
+                vals[o++] = i;
+            }
+    }
+}
+
+// Run boundaries of the sorted keys: [begin, end) for every tile that has
+// samples (both stay 0 for the others).
+__global__ void __launch_bounds__(256) k_tile_bounds(const uint32_t* __restrict__ keys,
+                                                     const uint32_t* __restrict__ dCount,
+                                                     uint2* __restrict__ tiles) {
+    const uint32_t n = *dCount;
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const uint32_t k = keys[i];
+        if (i == 0 || keys[i - 1] != k) tiles[k].x = i;
+        if (i + 1 == n || keys[i + 1] != k) tiles[k].y = i + 1;
+    }
+}
+
+// KCFilterToImgBlock / KCFilterToImgWarp (GPUReconFilterKC.cuh:146-377): a warp
+// per 8 x 4 pixels.  It reads its tile's samples 32 at a time, one per lane, and
+// keeps those whose window touches its pixels; then it takes these in order from
+// shared memory, every lane holding the sample against its own pixel.  So a pixel
+// sums its samples in ascending order, whatever their number.  Bound by the reads
+// of ids and coordinates, hence the two rounds ahead, and where samples crowd by
+// the steps of one warp per tile.  1M samples, 1080p, tent of radius 1, whole
+// splat: 341 us by pairs, 240 us so; 20,000 samples in one pixel: 2,500 us and 1,120.
+// Tiles of 16 x 16 (1.3 entries per sample instead of 1.6): 250 us and 2,770.
+template <int C, int kType>
+__global__ void __launch_bounds__(256) k_filter_tiles(
+    const uint2* __restrict__ tiles, int32_t tilesX, const uint32_t* __restrict__ vals,
+    const float* __restrict__ values, const float2* __restrict__ coords, ReconFilterDev f,
+    ImageSeg g, float multiplier, float* __restrict__ pixels, float* __restrict__ counts) {
+    constexpr uint32_t kAll = 0xFFFFFFFFu;
+    __shared__ float4 place[8][32];  // coordinates, the window's first pixel
+    __shared__ __align__(16) float value[8][32][C];
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    // the warp's and the lane's pixel, in the segment
+    const int32_t blocksX = (tilesX + 1) / 2;
+    const int32_t wx = (int32_t(blockIdx.x) % blocksX) * 16 + int32_t(warp & 1u) * 8;
+    const int32_t wy = (int32_t(blockIdx.x) / blocksX) * 16 + int32_t(warp >> 1) * 4;
+    if (wx >= g.w || wy >= g.h) return;
+    const uint2 range = tiles[(wy / kTileSide) * tilesX + wx / kTileSide];
+    if (range.x == range.y) return;
+    f.type = kType;
+    const int32_t qx = wx + int32_t(lane & 7u), qy = wy + int32_t(lane >> 3);
+    const int32_t gx = qx + g.offX, gy = qy + g.offY;
+    const float pcx = static_cast<float>(gx) + 0.5f, pcy = static_cast<float>(gy) + 0.5f;
+    // a window of one pixel reaches it wherever the sample lies in it
+    const float r2 = f.wh == 1u ? INFINITY : f.radius * f.radius;
+    const SamplePix any = sample_pix(0.5f, 0.5f, f.wh);
+    const int32_t extent = any.x1 - any.x0;  // of a window, per axis
+    float acc[C];
+    for (int k = 0; k < C; k++) acc[k] = 0.0f;
+    float wsum = 0.0f;
+    bool hit = false;
+    // ids are read two rounds ahead and coordinates one
+    auto id_at = [&](uint32_t i) { return i < range.y ? __ldg(vals + i) : 0u; };
+    auto coord_at = [&](uint32_t i, uint32_t id) {
+        return i < range.y ? __ldg(coords + id) : make_float2(0.0f, 0.0f);
+    };
+    uint32_t id = id_at(range.x + lane), id1 = id_at(range.x + 32u + lane);
+    float2 c = coord_at(range.x + lane, id);
+    for (uint32_t base = range.x; base < range.y; base += 32u) {
+        const uint32_t i = base + lane;
+        const uint32_t id2 = id_at(i + 64u);
+        const float2 c1 = coord_at(i + 32u, id1);
+        int32_t lowX = 0, lowY = 0;
+        bool touches = false;
+        if (i < range.y) {
+            const SamplePix s = sample_pix(c.x, c.y, f.wh);
+            lowX = s.ix + s.x0;
+            lowY = s.iy + s.y0;
+            const int32_t dx = wx + g.offX - lowX, dy = wy + g.offY - lowY;
+            touches = dx > -8 && dx < extent && dy > -4 && dy < extent;
+        }
+        const uint32_t some = __ballot_sync(kAll, touches);
+        if (touches) {
+            const uint32_t at = uint32_t(__popc(some & ((1u << lane) - 1u)));
+            place[warp][at] = make_float4(c.x, c.y, __int_as_float(lowX), __int_as_float(lowY));
+            if constexpr (C == 4)
+                *reinterpret_cast<float4*>(value[warp][at]) =
+                    reinterpret_cast<const float4*>(values)[id];
+            else
+                value[warp][at][0] = values[id];
+        }
+        __syncwarp();
+        const int count = __popc(some);
+#pragma unroll 4
+        for (int h = 0; h < count; h++) {
+            const float4 s = place[warp][h];
+            const float dx = s.x - pcx, dy = s.y - pcy;
+            const bool reaches =
+                (uint32_t(gx - __float_as_int(s.z)) < uint32_t(extent)) &
+                (uint32_t(gy - __float_as_int(s.w)) < uint32_t(extent)) &
+                ((dx * dx + dy * dy) <= r2);
+            float w = 0.0f;
+            if (kType <= kReconTent || reaches) w = recon_weight(f, pcx, pcy, s.x, s.y) * multiplier;
+            wsum = reaches ? wsum + w : wsum;
+            for (int k = 0; k < C; k++)
+                acc[k] = reaches ? acc[k] + w * value[warp][h][k] : acc[k];
+            hit |= reaches;
+        }
+        __syncwarp();
+        id = id1;
+        id1 = id2;
+        c = c1;
+    }
+    // a tile may stick out of the segment and a segment out of the image
+    if (!hit || qx >= g.w || qy >= g.h || !in_segment(g, gx, gy)) return;
+    const size_t q = size_t(qy) * size_t(g.w) + size_t(qx);
+    if constexpr (C == 4) {
+        float4* p4 = reinterpret_cast<float4*>(pixels) + q;
+        float4 p = *p4;
+        p.x += acc[0];
+        p.y += acc[1];
+        p.z += acc[2];
+        p.w += acc[3];
+        *p4 = p;
+    } else {
+        pixels[q] += acc[0];
+    }
+    counts[q] += wsum;
 }
 
 // Tracer splat over the camera's sample grid.  Sample sid = sy * (W*sp) + sx
@@ -412,67 +587,82 @@ int recon_filter_make(const char* type, float radius, uint32_t optCount, const c
     return 0;
 }
 
-static size_t pair_capacity(const ReconFilterDev& f, uint32_t n) {
-    return size_t(n) * f.wh * f.wh;
+// Most tiles that a sample's window touches.
+static uint32_t tiles_per_sample(const ReconFilterDev& f) {
+    const uint32_t axis = (f.wh + uint32_t(kTileSide) - 2u) / uint32_t(kTileSide) + 1u;
+    return axis * axis;
+}
+static uint32_t tile_columns(const ImageSeg& seg) {
+    return uint32_t(seg.w - 1) / uint32_t(kTileSide) + 1u;
+}
+static uint32_t tile_total(const ImageSeg& seg) {
+    return tile_columns(seg) * (uint32_t(seg.h - 1) / uint32_t(kTileSide) + 1u);
+}
+
+// Whether a splat lists samples by tile or by pixel.  A sample reaches pi r^2
+// pixels and touches (1 + (wh - 1) / 8)^2 tiles on average: 3.1 and 1.6 with a
+// radius of 1 (a window of 3), 0.8 and 1.3 with 0.5 (of 2).  Radius 1, 1M samples on 1080p
+// by tiles 233 us, by pairs 343; radius 2, 660,000 samples 229 and 660; radius 0.75
+// (the first of window 3) even; radius 0.5, 2.6M samples 410 and 304.
+static bool use_tiles(const ReconFilterDev& f) { return f.wh >= 3u; }
+
+// Carves the scratch of a splat out of base (null: only adds up its bytes).
+static size_t carve(unsigned char* base, const ReconFilterDev& f, uint32_t n, const ImageSeg& seg,
+                    ReconScratch& s) {
+    size_t at = 0;
+    auto take = [&](size_t bytes) {
+        unsigned char* p = base ? base + at : nullptr;
+        at += align256(bytes);
+        return p;
+    };
+    const bool tiles = use_tiles(f);
+    const size_t entries = size_t(n) * (tiles ? tiles_per_sample(f) : f.wh * f.wh);
+    const size_t lists = tiles ? tile_total(seg) : size_t(seg.w) * size_t(seg.h);
+    s.count = reinterpret_cast<uint32_t*>(take((size_t(n) + 1) * 4));
+    s.offset = reinterpret_cast<uint32_t*>(take((size_t(n) + 1) * 4));
+    s.scanTemp = take(exclusive_scan_temp_bytes(n));
+    s.keys = reinterpret_cast<uint32_t*>(take(entries * 4));
+    s.vals = reinterpret_cast<uint32_t*>(take(entries * 4));
+    s.entries = static_cast<uint32_t>(entries);
+    s.bits = key_bits(static_cast<uint32_t>(lists));
+    s.sortTempBytes = radix_sort_temp_bytes(s.entries, 4, 0, s.bits);
+    s.sortTemp = take(s.sortTempBytes);
+    if (tiles) {
+        s.tiles = reinterpret_cast<uint2*>(take(lists * 8));
+    } else {
+        s.begin = reinterpret_cast<uint32_t*>(take(lists * 4));
+        s.end = reinterpret_cast<uint32_t*>(take(lists * 4));
+    }
+    return at;
 }
 
 size_t recon_scratch_bytes(const ReconFilterDev& f, uint32_t n, const ImageSeg& seg) {
-    const size_t pairs = pair_capacity(f, n);
-    const size_t pix = size_t(seg.w) * size_t(seg.h);
-    const int bits = key_bits(static_cast<uint32_t>(pix));
-    size_t b = 0;
-    b += align256((size_t(n) + 1) * 4) * 2;
-    b += align256(exclusive_scan_temp_bytes(n));
-    b += align256(pairs * 4) * 2;
-    b += align256(radix_sort_temp_bytes(static_cast<uint32_t>(pairs), 4, 0, bits));
-    b += align256(pix * 4) * 2;
-    return b;
+    ReconScratch s{};
+    return carve(nullptr, f, n, seg, s);
 }
 
 ReconScratch recon_scratch_carve(void* base, const ReconFilterDev& f, uint32_t n,
                                  const ImageSeg& seg) {
-    const size_t pairs = pair_capacity(f, n);
-    const size_t pix = size_t(seg.w) * size_t(seg.h);
-    const int bits = key_bits(static_cast<uint32_t>(pix));
-    unsigned char* p = static_cast<unsigned char*>(base);
     ReconScratch s{};
-    s.count = reinterpret_cast<uint32_t*>(p);
-    p += align256((size_t(n) + 1) * 4);
-    s.offset = reinterpret_cast<uint32_t*>(p);
-    p += align256((size_t(n) + 1) * 4);
-    s.scanTemp = p;
-    p += align256(exclusive_scan_temp_bytes(n));
-    s.keys = reinterpret_cast<uint32_t*>(p);
-    p += align256(pairs * 4);
-    s.vals = reinterpret_cast<uint32_t*>(p);
-    p += align256(pairs * 4);
-    s.sortTemp = p;
-    s.sortTempBytes = radix_sort_temp_bytes(static_cast<uint32_t>(pairs), 4, 0, bits);
-    p += align256(s.sortTempBytes);
-    s.begin = reinterpret_cast<uint32_t*>(p);
-    p += align256(pix * 4);
-    s.end = reinterpret_cast<uint32_t*>(p);
+    carve(static_cast<unsigned char*>(base), f, n, seg, s);
     return s;
 }
 
-int recon_filter_to_img(const ReconFilterDev& f, const ImageSeg& seg, const float* values,
-                        uint32_t channels, const float2* coords, uint32_t n, float multiplier,
-                        float* pixels, float* counts, const ReconScratch& s, cudaStream_t stream) {
-    if (n == 0 || seg.w <= 0 || seg.h <= 0) return 0;
-    const size_t pairs = pair_capacity(f, n);
+static int splat_pairs(const ReconFilterDev& f, const ImageSeg& seg, const float* values,
+                       uint32_t channels, const float2* coords, uint32_t n, float multiplier,
+                       float* pixels, float* counts, const ReconScratch& s, cudaStream_t stream) {
     const size_t pix = size_t(seg.w) * size_t(seg.h);
-    const int bits = key_bits(static_cast<uint32_t>(pix));
     const uint32_t g = grid_of(n, 148 * 8);
     k_expand_count<<<g, 256, 0, stream>>>(coords, n, f, seg, s.count);
     if (exclusive_scan_u32(s.count, s.offset, n, s.scanTemp, stream)) return MRB_E_CUDA;
     k_expand_write<<<g, 256, 0, stream>>>(coords, n, f, seg, s.offset, s.keys, s.vals);
     const uint32_t* dTotal = s.offset + n;
-    if (radix_sort_pairs<uint32_t>(s.keys, s.vals, dTotal, static_cast<uint32_t>(pairs), 0, bits,
-                                   false, s.sortTemp, s.sortTempBytes, stream, false))
+    if (radix_sort_pairs<uint32_t>(s.keys, s.vals, dTotal, s.entries, 0, s.bits, false, s.sortTemp,
+                                   s.sortTempBytes, stream, false))
         return MRB_E_CUDA;
     MRB_CUDA(cudaMemsetAsync(s.begin, 0, pix * 4, stream));
     MRB_CUDA(cudaMemsetAsync(s.end, 0, pix * 4, stream));
-    k_pixel_bounds<<<grid_of(pairs, 148 * 8), 256, 0, stream>>>(s.keys, dTotal, s.begin, s.end);
+    k_pixel_bounds<<<grid_of(s.entries, 148 * 8), 256, 0, stream>>>(s.keys, dTotal, s.begin, s.end);
     const uint32_t gp = grid_of(pix, 148 * 16);
     if (channels == 4)
         k_filter_pixels<4><<<gp, 256, 0, stream>>>(s.begin, s.end, s.vals, values, coords, f, seg,
@@ -482,6 +672,49 @@ int recon_filter_to_img(const ReconFilterDev& f, const ImageSeg& seg, const floa
                                                    multiplier, pixels, counts);
     MRB_CUDA(cudaGetLastError());
     return 0;
+}
+
+static int splat_tiles(const ReconFilterDev& f, const ImageSeg& seg, const float* values,
+                       uint32_t channels, const float2* coords, uint32_t n, float multiplier,
+                       float* pixels, float* counts, const ReconScratch& s, cudaStream_t stream) {
+    const int32_t columns = static_cast<int32_t>(tile_columns(seg));
+    const uint32_t g = grid_of(n, 148 * 8);
+    k_tile_count<<<g, 256, 0, stream>>>(coords, n, f.wh, seg, s.count);
+    if (exclusive_scan_u32(s.count, s.offset, n, s.scanTemp, stream)) return MRB_E_CUDA;
+    k_tile_write<<<g, 256, 0, stream>>>(coords, n, f.wh, seg, columns, s.offset, s.keys, s.vals);
+    const uint32_t* dTotal = s.offset + n;
+    if (radix_sort_pairs<uint32_t>(s.keys, s.vals, dTotal, s.entries, 0, s.bits, false, s.sortTemp,
+                                   s.sortTempBytes, stream, false))
+        return MRB_E_CUDA;
+    MRB_CUDA(cudaMemsetAsync(s.tiles, 0, size_t(tile_total(seg)) * 8, stream));
+    k_tile_bounds<<<grid_of(s.entries, 148 * 8), 256, 0, stream>>>(s.keys, dTotal, s.tiles);
+    const uint32_t blocks = (uint32_t(seg.w - 1) / 16u + 1u) * (uint32_t(seg.h - 1) / 16u + 1u);
+    auto launch = [&](auto ch, auto type) {
+        k_filter_tiles<decltype(ch)::value, decltype(type)::value><<<blocks, 256, 0, stream>>>(
+            s.tiles, columns, s.vals, values, coords, f, seg, multiplier, pixels, counts);
+    };
+    auto of_type = [&](auto ch) {
+        switch (f.type) {
+            case kReconBox: launch(ch, std::integral_constant<int, kReconBox>{}); break;
+            case kReconTent: launch(ch, std::integral_constant<int, kReconTent>{}); break;
+            case kReconGaussian: launch(ch, std::integral_constant<int, kReconGaussian>{}); break;
+            default: launch(ch, std::integral_constant<int, kReconMitchell>{}); break;
+        }
+    };
+    if (channels == 4) of_type(std::integral_constant<int, 4>{});
+    else of_type(std::integral_constant<int, 1>{});
+    MRB_CUDA(cudaGetLastError());
+    return 0;
+}
+
+int recon_filter_to_img(const ReconFilterDev& f, const ImageSeg& seg, const float* values,
+                        uint32_t channels, const float2* coords, uint32_t n, float multiplier,
+                        float* pixels, float* counts, const ReconScratch& s, cudaStream_t stream) {
+    if (n == 0 || seg.w <= 0 || seg.h <= 0) return 0;
+    return use_tiles(f) ? splat_tiles(f, seg, values, channels, coords, n, multiplier, pixels,
+                                      counts, s, stream)
+                        : splat_pairs(f, seg, values, channels, coords, n, multiplier, pixels,
+                                      counts, s, stream);
 }
 
 int recon_filter_grid(const ReconFilterDev& f, const float4* samples, const float2* coords,

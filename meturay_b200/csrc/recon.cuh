@@ -91,18 +91,21 @@ int recon_filter_make(const char* type, float radius, uint32_t optCount, const c
                       const float* values, ReconFilterDev* out);
 
 // General splat of arbitrary (value, image coordinate) samples: the
-// expand -> sort-by-pixel -> per-pixel reduction of FilterToImgInternal.
+// expand -> sort -> per-pixel reduction of FilterToImgInternal.
 // channels: 1 (float values, R image) or 4 (float4 values, RGBA image).
 struct ReconScratch {
     uint32_t* count;      // n + 1
     uint32_t* offset;     // n + 1
     void* scanTemp;
-    uint32_t* keys;       // n * wh^2
-    uint32_t* vals;       // n * wh^2
+    uint32_t* keys;       // entries
+    uint32_t* vals;       // entries
+    uint32_t entries;     // most pairs, or tiles of samples, of any n samples
+    int bits;             // of a key
     void* sortTemp;
     size_t sortTempBytes;
-    uint32_t* begin;      // segment pixels
-    uint32_t* end;        // segment pixels
+    uint32_t* begin;      // segment pixels (pairs)
+    uint32_t* end;        // segment pixels (pairs)
+    uint2* tiles;         // per tile of the segment: its run [x, y)
 };
 size_t recon_scratch_bytes(const ReconFilterDev& f, uint32_t n, const ImageSeg& seg);
 ReconScratch recon_scratch_carve(void* base, const ReconFilterDev& f, uint32_t n,

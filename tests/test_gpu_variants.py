@@ -171,3 +171,58 @@ def test_ploc_steps_and_areas(system, cuda, n):
     assert abs(info["inner_area_ploc"] - area) <= n * 2.0 ** -52 * area
     g.construct_accelerators()  # again over the built scene
     assert g.accel_info()["ploc_steps"] == steps
+
+
+
+
+# ---- reconstruction splat ----------------------------------------------------
+def _bits_equal(a, b):
+    return np.array_equal(np.asarray(a, np.float32).view(np.uint32),
+                          np.asarray(b, np.float32).view(np.uint32))
+
+
+def _splat(torch, ftype, radius, params, values, coords, res, segment=None):
+    import meturay_b200 as m
+    img = m.ImageMemory(res[0], res[1], 1 if values.ndim == 1 else 4)
+    if segment is not None:
+        ox, oy, w, h = segment
+        img.reportion((ox, oy), (ox + w, oy + h))
+    m.ReconFilter(ftype, radius, params).filter_to_img(img, _dev(torch, values),
+                                                       _dev(torch, coords), coords.shape[0])
+    torch.cuda.synchronize()
+    return img.get_image()
+
+
+# windows of 1 and 2 pixels (pairs), of 3 to 5 (tiles), and one wider than a tile of the sorted lists
+@pytest.mark.parametrize("ftype,radius,params", [
+    ("Box", 0.0, {}), ("Box", 0.25, {}), ("Box", 0.5, {}), ("Tent", 0.75, {}), ("Tent", 1.0, {}),
+    ("Gaussian", 1.25, {"alpha": 1.0}), ("Mitchell", 2.0, {"b": 1 / 3, "c": 1 / 3}),
+    ("Tent", 9.25, {})])
+@pytest.mark.parametrize("channels", [1, 4])
+def test_splat_windows_at_image_edges(cuda, oracle, ftype, radius, params, channels):
+    rng = np.random.default_rng(int(radius * 100) + channels)
+    n, w, h = 9000, 67, 41
+    coords = np.stack([rng.uniform(-4, w + 4, n), rng.uniform(-4, h + 4, n)], 1).astype(np.float32)
+    coords[:6] = [[0, 0], [w, h], [np.nan, 3], [3, np.inf], [2e9, 1], [-0.5, -0.5]]
+    values = rng.uniform(0, 8, (n, channels)).astype(np.float32)
+    values = values if channels == 4 else values[:, 0]
+    seg = (5, 3, 50, 30)
+    px, cnt = _splat(cuda, ftype, radius, params, values, coords, (w, h), seg)
+    rp, rc = oracle.filter_to_img(ftype, radius, values, coords, (w, h), segment=seg, **params)
+    assert _bits_equal(px, rp) and _bits_equal(cnt, rc)
+
+
+def test_splat_of_crowded_pixels(cuda, oracle):
+    """From none to hundreds of samples at a pixel; each pixel's sum is in the
+    samples' order, so the bits are the oracle's."""
+    rng = np.random.default_rng(8)
+    w, h = 200, 150
+    spots = [(20.5, 30.5, 9), (60.2, 70.9, 40), (120.0, 100.0, 700), (199.9, 149.9, 90)]
+    coords = [np.array([x, y]) + rng.uniform(-1.2, 1.2, (k, 2)) for x, y, k in spots]
+    coords.append(np.stack([rng.uniform(0, w, 3000), rng.uniform(0, h, 3000)], 1))
+    coords = rng.permutation(np.concatenate(coords)).astype(np.float32)
+    values = rng.uniform(0, 4, (len(coords), 4)).astype(np.float32)
+    for ftype, radius, params in (("Tent", 1.0, {}), ("Gaussian", 2.0, {"alpha": 0.5})):
+        px, cnt = _splat(cuda, ftype, radius, params, values, coords, (w, h))
+        rp, rc = oracle.filter_to_img(ftype, radius, values, coords, (w, h), **params)
+        assert _bits_equal(px, rp) and _bits_equal(cnt, rc)
