@@ -185,7 +185,8 @@ int record_iteration(mrb_pool* p) {
         if ((r = trace_closest_wide_jobs(p->devJobs(), p->aux[cur].as<RayAux>(),
                                          p->rayO[cur].as<float4>(), p->rayD[cur].as<float4>(),
                                          cnt + cur, p->maxRays, ho,
-                                         p->errorFlags.as<uint32_t>(), p->block, p->stack, st)))
+                                         p->errorFlags.as<uint32_t>(), p->block, p->stack,
+                                         d > 0, st)))
             return r;
         // also adds this wavefront to the traced-ray total and clears the
         // next wavefront's counter

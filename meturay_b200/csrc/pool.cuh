@@ -53,6 +53,6 @@ int shade_jobs(const JobDev* jobs, const float4* rayO, const float4* rayD, const
 int trace_closest_wide_jobs(const JobDev* jobs, const RayAux* aux, const float4* rayO,
                             const float4* rayD, const uint32_t* dCount, uint32_t maxCount,
                             const HitOut& out, uint32_t* errorFlag, int block, int stack,
-                            cudaStream_t stream);
+                            bool refill, cudaStream_t stream);
 
 }  // namespace mrb
