@@ -33,6 +33,17 @@ constexpr float kFltMax = 3.40282347e+38f;
 // Ray types (RayAuxStruct.cuh RayType)
 constexpr uint8_t kNeeRay = 0, kSpecPathRay = 1, kPathRay = 2, kCameraRay = 3;
 constexpr uint32_t kTagCamera = 0x10000u;
+// tMin of a plain tracer's next-event ray to light `light`, which it names to the
+// traversal (HitOut::shadowRays): minus a subnormal number with the light in its
+// bits, which no hit distance (over 1e-7) lies below.  Lights beyond its 23 bits
+// are not named.
+__host__ __device__ __forceinline__ float shadow_tmin(uint32_t light) {
+    union { uint32_t u; float f; } v{light < (1u << 23) ? 0x80000000u | light : 0u};
+    return v.f;
+}
+__host__ __device__ __forceinline__ bool is_shadow_tmin(uint32_t bits) {
+    return (bits >> 23) == 0x100u;
+}
 
 // ---------------------------------------------------------------------------
 // Device-resident layouts

@@ -181,7 +181,7 @@ int record_iteration(mrb_pool* p) {
     for (uint32_t d = 0; d < p->maxDepth; d++) {
         const int cur = d & 1, nxt = cur ^ 1;
         const HitOut ho{p->hitKey.as<uint32_t>(), p->hitPrim.as<uint32_t>(), p->hitT.as<float>(),
-                        p->hitBary.as<float2>()};
+                        p->hitBary.as<float2>(), true};
         if ((r = trace_closest_wide_jobs(p->devJobs(), p->aux[cur].as<RayAux>(),
                                          p->rayO[cur].as<float4>(), p->rayD[cur].as<float4>(),
                                          cnt + cur, p->maxRays, ho,

@@ -689,7 +689,7 @@ int step_depth(mrb_tracer* t, uint32_t d, StageTimer* tm = nullptr,
     const int cur = d & 1, nxt = cur ^ 1;
     uint32_t* cnt = t->count.as<uint32_t>();
     HitOut ho{t->hitKey.as<uint32_t>(), t->hitPrim.as<uint32_t>(), t->hitT.as<float>(),
-              t->hitBary.as<float2>()};
+              t->hitBary.as<float2>(), !t->wfpg};
     int r;
     auto mark = [&](int i) -> int {
         if (tm) MRB_CUDA(cudaEventRecord(tm->ev[i], t->stream));

@@ -324,7 +324,7 @@ __global__ void __launch_bounds__(kShadeBlock, 6) k_shade(ShadeArgs A) {
                     if (nonzero(nrf)) {
                         const V3 o = nudge(sf.pos, sf.geo);
                         emitNee = true;
-                        neeO = make_float4(o.x, o.y, o.z, 0.0f);
+                        neeO = make_float4(o.x, o.y, o.z, A.opt.wfpg ? 0.0f : shadow_tmin(li));
                         neeD = make_float4(ldir.x, ldir.y, ldir.z, kFltMax);
                         neeAux = aux;
                         neeAux.rf[0] = nrf.x;

@@ -11,6 +11,9 @@ struct HitOut {
     uint32_t* prim;  // original triangle index, 0xFFFFFFFF on a miss
     float* t;        // hit distance (tMax when missed)
     float2* bary;    // (1-u-v, u) as the reference's TriangleHit
+    // Rays with a tMin of shadow_tmin are shadow rays: the 8-wide kernels report
+    // a miss where their light is not the closest hit.
+    bool shadowRays = false;
 };
 
 // rayO[i] = (origin, tMin), rayD[i] = (direction, tMax).

@@ -784,10 +784,25 @@ __device__ __forceinline__ void trace_wide_ray(const WideAccelDev& acc, const Wi
     }
 }
 
+// A next-event ray of a plain tracer that something stops brings no radiance, so
+// it is reported as a miss and shading skips it: half of closed Cornell's hits
+// (1080p, four samples per pixel, five depths: shading 3.99 -> 3.15 ms per frame).
+// The WFPG tracer counts what stopped its rays and marks none.  Stopping
+// the traversal at the first triangle nearer than the light was tried: the test
+// in the node loops cost more (11.4 -> 11.6 ms; open scenes 3 %) than it saved.
 __device__ __forceinline__ void write_hit(const WideAccelDev& acc, const HitOut& out, uint32_t i,
-                                          int hitTri, float closest, float hb0, float hb1) {
+                                          float tmin, int hitTri, float closest, float hb0,
+                                          float hb1) {
+    uint32_t key = kBatchNull;
     if (hitTri >= 0) {
-        out.key[i] = __float_as_uint(__ldg(&acc.te0[hitTri].w));
+        key = __float_as_uint(__ldg(&acc.te0[hitTri].w));
+        const uint32_t mark = __float_as_uint(tmin);
+        if (out.shadowRays && is_shadow_tmin(mark) &&
+            key != ((kBatchLight << kIdBits) | (mark & 0x7FFFFFu)))
+            key = kBatchNull;
+    }
+    if (key != kBatchNull) {
+        out.key[i] = key;
         out.prim[i] = __float_as_uint(__ldg(&acc.tv0[hitTri].w));
         out.t[i] = closest;
         out.bary[i] = make_float2(hb0, hb1);
@@ -842,7 +857,7 @@ __global__ void __launch_bounds__(128, 8) k_trace_wide(WideAccelDev acc,
         WideRay r;
         trace_wide_ray<kCount, kOctant, WideStack<kOctant>::value>(
             acc, sNodes, cached, rayO[i], rayD[i], r, nodeVisits, triTests, errorFlag);
-        write_hit(acc, out, i, r.hitTri, r.closest, r.hb0, r.hb1);
+        write_hit(acc, out, i, r.tmin, r.hitTri, r.closest, r.hb0, r.hb1);
     }
     if (kCount) add_work(counters, nodeVisits, triTests);
 }
@@ -878,7 +893,7 @@ __global__ void __launch_bounds__(128, 8) k_trace_wide_refill(WideAccelDev acc,
             WideRay r;
             trace_wide_ray<kCount, kOctant, kStack>(acc, sNodes, cached, rayO[i], rayD[i], r,
                                                     nodeVisits, triTests, errorFlag);
-            write_hit(acc, out, i, r.hitTri, r.closest, r.hb0, r.hb1);
+            write_hit(acc, out, i, r.tmin, r.hitTri, r.closest, r.hb0, r.hb1);
         }
     } else {
         const uint32_t lane = threadIdx.x & 31u;
@@ -911,7 +926,7 @@ __global__ void __launch_bounds__(128, 8) k_trace_wide_refill(WideAccelDev acc,
             if (!active) continue;
             if (!wide_visit<kCount, kOctant, kStack>(acc, sNodes, cached, r, stack, nodeVisits,
                                                      triTests, errorFlag)) {
-                write_hit(acc, out, ri, r.hitTri, r.closest, r.hb0, r.hb1);
+                write_hit(acc, out, ri, r.tmin, r.hitTri, r.closest, r.hb0, r.hb1);
                 active = false;
             }
         }
@@ -940,7 +955,7 @@ __global__ void __launch_bounds__(kBlock, 1024 / kBlock) k_trace_wide_jobs(
             WideRay r;
             trace_wide_ray<false, kOctant, kEntries>(acc, nullptr, 0, rayO[i], rayD[i], r,
                                                      nodeVisits, triTests, errorFlag);
-            write_hit(acc, out, i, r.hitTri, r.closest, r.hb0, r.hb1);
+            write_hit(acc, out, i, r.tmin, r.hitTri, r.closest, r.hb0, r.hb1);
         }
     } else {
         const uint32_t lane = threadIdx.x & 31u;
@@ -980,7 +995,7 @@ __global__ void __launch_bounds__(kBlock, 1024 / kBlock) k_trace_wide_jobs(
             else if (acc.triCount == 1)
                 tri_test(acc, 0, r.o, r.d, r.tmin, r.closest, r.hitTri, r.hb0, r.hb1);
             if (!going) {
-                write_hit(acc, out, ri, r.hitTri, r.closest, r.hb0, r.hb1);
+                write_hit(acc, out, ri, r.tmin, r.hitTri, r.closest, r.hb0, r.hb1);
                 active = false;
             }
         }

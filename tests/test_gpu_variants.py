@@ -226,3 +226,34 @@ def test_splat_of_crowded_pixels(cuda, oracle):
         px, cnt = _splat(cuda, ftype, radius, params, values, coords, (w, h))
         rp, rc = oracle.filter_to_img(ftype, radius, values, coords, (w, h), **params)
         assert _bits_equal(px, rp) and _bits_equal(cnt, rc)
+
+
+# ---- shadow rays -------------------------------------------------------------
+@pytest.mark.parametrize("order", range(4))
+@pytest.mark.parametrize("shielded,mis", [(False, 1), (True, 0)])
+def test_shadow_rays_see_what_the_binary_traversal_sees(system, cuda, order, shielded, mis):
+    """The 8-wide kernels report a next-event ray that its light's triangle does
+    not end as a miss, the binary traversal reports what it hit.  Both run the
+    same triangle test, so pixels differ by the order of their sums (a few ulp)
+    but for paths that pass through two triangles at the same distance."""
+    import meturay_b200 as m
+    g = m.GPUScene(system, m.scenes.cornell(seed=1, shielded=shielded))
+    g.construct_accelerators()
+
+    def image(traversal):
+        g.set_traversal(traversal)
+        t = m.PathTracer(system, g)
+        t.set_options({"Samples": 2, "MaxDepth": 4, "NextEventEstimation": 1,
+                       "DirectLightMIS": mis, "RussianRouletteStart": 3, "Seed": 7})
+        t.set_resolution(160, 120)
+        for _ in range(4):
+            t.render_frame()
+        out = np.array(t.image())
+        t.close()
+        return out
+
+    g.set_wide_order(order)
+    wide, binary = image(1), image(0)
+    assert wide[..., :3].sum() > 0
+    differ = (np.abs(wide - binary) > 1e-5 * (1.0 + np.abs(binary))).any(-1)
+    assert differ.mean() < 2e-3
