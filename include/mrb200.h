@@ -155,8 +155,9 @@ int mrb_accel_info(const mrb_scene* scene, uint32_t* info4);
  * built), then per depth on a tracer's own rays: the frame that
  * mrb_tracer_render_frame runs before it captures its graph traces every
  * depth's rays with every kernel and keeps the fastest per depth (once per
- * tracer and traversal setting).  Closest hits are the same with every
- * kernel, up to the choice among triangles at the same distance. */
+ * tracer and traversal setting); mrb_accel_hit traces up to 32,768 rays with
+ * a warp each.  Closest hits are the same with every kernel, up to the choice
+ * among triangles at the same distance. */
 #define MRB_WIDE_SORTED 0
 #define MRB_WIDE_OCTANT 1
 #define MRB_WIDE_SORTED_REFILL 2

@@ -934,6 +934,123 @@ __global__ void __launch_bounds__(128, 8) k_trace_wide_refill(WideAccelDev acc,
     if (kCount) add_work(counters, nodeVisits, triTests);
 }
 
+// ---------------------------------------------------------------------------
+// One warp per ray, for a few thousand rays
+// ---------------------------------------------------------------------------
+// With one lane per ray so few rays leave most schedulers a warp or none, and
+// the launch lasts as long as its longest ray's chain of node visits, each a
+// dependent read and eight box tests (2,000 rays over 1M triangles: 96 us).
+// Here a warp takes a ray: up to four pending nodes at a time, one per team of
+// eight lanes, one child slot per lane; the triangles of all hit leaves at once,
+// one per lane.  Lane k of a team has slot k ^ (ray octant), so that lower lanes
+// are nearer and the hits are pushed to be taken in that order, the top node's
+// first.  Entries keep their distance and are dropped once a nearer hit is
+// known.  The nodes taken beside the top one are speculative; what they cost
+// is idle hardware here, which is why larger launches trace with one lane per
+// ray.  The fastest of those kernels and this one, clusters 1M and Cornell: 2,000
+// rays 97 and 24 us, 41 and 13; 16,000 rays 103 and 60, 58 and 27; 32,000 rays 110
+// and 102, 60 and 46; the same at 64,000 (hence kWideWarpRays).
+constexpr int kWarpStack = 256;       // entries per warp
+constexpr int kWarpBlock = 128;
+
+__global__ void __launch_bounds__(kWarpBlock) k_trace_wide_warp(
+    WideAccelDev acc, const float4* __restrict__ rayO, const float4* __restrict__ rayD, uint32_t n,
+    HitOut out, uint32_t* errorFlag) {
+    constexpr uint32_t kAll = 0xFFFFFFFFu;
+    __shared__ uint2 stacks[kWarpBlock / 32][kWarpStack];
+    const uint32_t lane = threadIdx.x & 31u, team = lane >> 3;
+    uint2* stack = stacks[threadIdx.x >> 5];
+    const uint32_t warps = (gridDim.x * kWarpBlock) >> 5;
+    uint32_t nodeVisits = 0, triTests = 0;  // not asked for
+    for (uint32_t i = (blockIdx.x * kWarpBlock + threadIdx.x) >> 5; i < n; i += warps) {
+        WideRay r;
+        uint32_t owner = 0;
+        wide_ray_begin(r, rayO[i], rayD[i]);
+        const uint32_t slot = (lane & 7u) ^ r.oct;
+        int sp = 1;
+        __syncwarp();
+        if (lane == 0) stack[0] = make_uint2(0u, 0u);
+        __syncwarp();
+        while (sp > 0) {
+            // deep in the stack one node at a time, as a plain depth-first
+            // traversal, which adds at most seven entries per level
+            const int take = sp > kWarpStack / 2 ? 1 : min(sp, 4);
+            uint2 e = make_uint2(0u, 0u);
+            bool active = int(team) < take;
+            if (active) {
+                e = stack[sp - 1 - int(team)];
+                active = __uint_as_float(e.y) <= r.closest;
+            }
+            sp -= take;
+            bool inner = false, leaf = false;
+            uint32_t child = 0;
+            float tn = 0.0f;
+            if (active) {
+                const uint4* g = reinterpret_cast<const uint4*>(acc.nodes + e.x);
+                const uint8_t* q = reinterpret_cast<const uint8_t*>(g + 2) + slot;
+                const uint4 w0 = __ldg(g), w1 = __ldg(g + 1);
+                const float lx = float(__ldg(q)), ly = float(__ldg(q + 8)),
+                            lz = float(__ldg(q + 16)), hx = float(__ldg(q + 24)),
+                            hy = float(__ldg(q + 32)), hz = float(__ldg(q + 40));
+                const float ax = __uint_as_float((w0.w & 0xFFu) << 23) * r.inv.x;
+                const float ay = __uint_as_float(((w0.w >> 8) & 0xFFu) << 23) * r.inv.y;
+                const float az = __uint_as_float(((w0.w >> 16) & 0xFFu) << 23) * r.inv.z;
+                const float bx = (__uint_as_float(w0.x) - r.o.x) * r.inv.x;
+                const float by = (__uint_as_float(w0.y) - r.o.y) * r.inv.y;
+                const float bz = (__uint_as_float(w0.z) - r.o.z) * r.inv.z;
+                const bool px = !(r.oct & 1u), py = !(r.oct & 2u), pz = !(r.oct & 4u);
+                tn = fmaxf(fmaxf(__fmaf_rn(px ? lx : hx, ax, bx), __fmaf_rn(py ? ly : hy, ay, by)),
+                           fmaxf(__fmaf_rn(pz ? lz : hz, az, bz), r.tmin));
+                const float tf =
+                    fminf(fminf(__fmaf_rn(px ? hx : lx, ax, bx), __fmaf_rn(py ? hy : ly, ay, by)),
+                          fminf(__fmaf_rn(pz ? hz : lz, az, bz), r.closest));
+                if (tn <= tf) {
+                    const uint32_t imask = w0.w >> 24, below = (1u << slot) - 1u;
+                    inner = (imask >> slot) & 1u;
+                    leaf = (w1.z >> slot) & 1u;
+                    child = inner ? w1.x + uint32_t(__popc(imask & below))
+                                  : w1.y + uint32_t(__popc(w1.z & below));
+                }
+            }
+            if (__any_sync(kAll, leaf)) {
+                float t = r.closest, b0 = 0.0f, b1 = 0.0f;
+                int tri = -1;
+                if (leaf) tri_test(acc, child, r.o, r.d, r.tmin, t, tri, b0, b1);
+                // distances are positive: their bits order as they do
+                const uint32_t key = tri >= 0 ? __float_as_uint(t) : kAll;
+                const uint32_t best = __reduce_min_sync(kAll, key);
+                if (best != kAll) {
+                    owner = uint32_t(__ffs(int(__ballot_sync(kAll, key == best))) - 1);
+                    r.closest = __uint_as_float(best);
+                    if (lane == owner) {
+                        r.hitTri = tri;
+                        r.hb0 = b0;
+                        r.hb1 = b1;
+                    }
+                }
+            }
+            const uint32_t push = __ballot_sync(kAll, inner);
+            if (sp + __popc(push) > kWarpStack) {
+                // a tree deeper than any the builds make: this ray again, by
+                // one lane with the octant kernel's stack
+                if (lane == 0)
+                    trace_wide_ray<false, true, kWideGroups>(acc, nullptr, 0, rayO[i], rayD[i], r,
+                                                             nodeVisits, triTests, errorFlag);
+                owner = 0;
+                break;
+            }
+            // the first lane's child on top
+            if (inner)
+                stack[sp + __popc(push & ~((2u << lane) - 1u))] =
+                    make_uint2(child, __float_as_uint(tn));
+            sp += __popc(push);
+            __syncwarp();
+        }
+        if (lane == owner)
+            write_hit(acc, out, i, r.tmin, r.hitTri, r.closest, r.hb0, r.hb1);
+    }
+}
+
 // Rays of many scenes: each ray's tree is its job's (RayAux::pad is the job
 // slot).  No shared-memory top levels: neighbouring rays may use different
 // trees.  kRefill: as k_trace_wide_refill, a warp's idle lanes take its next
@@ -1075,6 +1192,15 @@ int wide_build(const WideBuildIn& in, WideNode* nodes, float4* tv0, float4* te0,
     }
     set_error("wide BVH: collapse did not finish");
     return MRB_E_DEVICE;
+}
+
+int trace_closest_wide_few(const WideAccelDev& acc, const float4* rayO, const float4* rayD,
+                           uint32_t n, const HitOut& out, uint32_t* errorFlag,
+                           cudaStream_t stream) {
+    k_trace_wide_warp<<<std::min((n + 3u) / 4u, 148u * 16u), kWarpBlock, 0, stream>>>(
+        acc, rayO, rayD, n, out, errorFlag);
+    MRB_CUDA(cudaGetLastError());
+    return 0;
 }
 
 int trace_closest_wide(const WideAccelDev& acc, const float4* rayO, const float4* rayD,

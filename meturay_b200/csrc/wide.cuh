@@ -67,6 +67,12 @@ int trace_closest_wide(const WideAccelDev& acc, const float4* rayO, const float4
                        const uint32_t* dCount, uint32_t maxCount, const HitOut& out,
                        uint32_t* errorFlag, cudaStream_t stream,
                        unsigned long long* counters = nullptr, int order = 0);
+// The same closest hits by a warp per ray, the faster form up to kWideWarpRays
+// (1 to kWideWarpRays rays over two triangles or more).
+constexpr uint32_t kWideWarpRays = 32768;
+int trace_closest_wide_few(const WideAccelDev& acc, const float4* rayO, const float4* rayD,
+                           uint32_t n, const HitOut& out, uint32_t* errorFlag,
+                           cudaStream_t stream);
 // Scratch of the two probes below.
 size_t wide_probe_bytes();
 // Bytes the octant kernel reads (node visits x 80 B + triangle tests x

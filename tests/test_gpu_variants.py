@@ -257,3 +257,41 @@ def test_shadow_rays_see_what_the_binary_traversal_sees(system, cuda, order, shi
     assert wide[..., :3].sum() > 0
     differ = (np.abs(wide - binary) > 1e-5 * (1.0 + np.abs(binary))).any(-1)
     assert differ.mean() < 2e-3
+
+
+# ---- few rays ----------------------------------------------------------------
+@pytest.mark.parametrize("name", ["clusters", "cornell"])
+@pytest.mark.parametrize("n", [1, 3, 4, 5, 2000, 32767, 32768, 32769])
+def test_few_rays_hit_what_a_lane_per_ray_hits(system, cuda, name, n):
+    """Up to 32,768 rays a warp traces each ray, with the same triangle test:
+    the distances are the same bits, and the triangles too but for ties."""
+    import meturay_b200 as m
+    torch = cuda
+    scene = m.scenes.clusters(1, n_clusters=40) if name == "clusters" else m.scenes.cornell(seed=1)
+    size = 100.0 if name == "clusters" else 1.0
+    g = m.GPUScene(system, scene)
+    g.construct_accelerators()
+    gen = torch.Generator(device="cuda").manual_seed(n)
+    o = torch.rand((n, 4), generator=gen, device="cuda") * size
+    d = torch.randn((n, 4), generator=gen, device="cuda")
+    d[:, :3] /= d[:, :3].norm(dim=1, keepdim=True)
+    d[::5, 0] = 0.0  # directions within a plane and along an axis
+    d[::10, 1] = 0.0
+    o[:, 3] = 0.0
+    d[:, 3] = 1000.0
+    d[::7, 3] = 0.05 * size  # short rays
+
+    def hits(order):
+        g.set_wide_order(order)
+        out = [torch.full((n,), -7, dtype=torch.int32, device="cuda") for _ in range(2)]
+        out += [torch.full((n,), -7.0, device="cuda"), torch.full((n, 2), -7.0, device="cuda")]
+        g.hit(o.data_ptr(), d.data_ptr(), n, *(x.data_ptr() for x in out))
+        torch.cuda.synchronize()
+        return out
+
+    few, lanes = hits("auto"), hits("sorted")
+    assert torch.equal(few[2], lanes[2])
+    same = few[1] == lanes[1]
+    assert int((~same).sum()) <= 1 + n // 1000
+    assert torch.equal(few[0][same], lanes[0][same])
+    assert torch.equal(few[3][same], lanes[3][same])
