@@ -601,10 +601,18 @@ static uint32_t tile_total(const ImageSeg& seg) {
 
 // Whether a splat lists samples by tile or by pixel.  A sample reaches pi r^2
 // pixels and touches (1 + (wh - 1) / 8)^2 tiles on average: 3.1 and 1.6 with a
-// radius of 1 (a window of 3), 0.8 and 1.3 with 0.5 (of 2).  Radius 1, 1M samples on 1080p
-// by tiles 233 us, by pairs 343; radius 2, 660,000 samples 229 and 660; radius 0.75
-// (the first of window 3) even; radius 0.5, 2.6M samples 410 and 304.
-static bool use_tiles(const ReconFilterDev& f) { return f.wh >= 3u; }
+// radius of 1 (a window of 3), 0.8 and 1.3 with 0.5 (of 2).  Radius 1, 1M samples
+// on 1080p: by tiles 233 us, by pairs 343; radius 0.5, 2.6M samples: 410 and 304.
+// Where many samples crowd on few tiles (over kDense reaching a pixel of an image
+// below kWide pixels) their warps' serial walks take longer than the sort of the
+// pairs: radius 1.33, 154,930 samples on 79 x 72 214 us and 182, radius 0.75, 16
+// reaching a pixel of 256 x 256 169 and 151; 16 with a radius of 1 112 and 145.
+static bool use_tiles(const ReconFilterDev& f, uint32_t n, const ImageSeg& seg) {
+    constexpr double kDense = 8.0, kWide = 65536.0;
+    const double pix = double(seg.w) * double(seg.h);
+    const bool dense = double(n) * 3.1416 * double(f.radius) * double(f.radius) > kDense * pix;
+    return f.wh >= 3u && (!dense || (pix >= kWide && f.radius >= 1.0f));
+}
 
 // Carves the scratch of a splat out of base (null: only adds up its bytes).
 static size_t carve(unsigned char* base, const ReconFilterDev& f, uint32_t n, const ImageSeg& seg,
@@ -615,7 +623,7 @@ static size_t carve(unsigned char* base, const ReconFilterDev& f, uint32_t n, co
         at += align256(bytes);
         return p;
     };
-    const bool tiles = use_tiles(f);
+    const bool tiles = use_tiles(f, n, seg);
     const size_t entries = size_t(n) * (tiles ? tiles_per_sample(f) : f.wh * f.wh);
     const size_t lists = tiles ? tile_total(seg) : size_t(seg.w) * size_t(seg.h);
     s.count = reinterpret_cast<uint32_t*>(take((size_t(n) + 1) * 4));
@@ -711,10 +719,8 @@ int recon_filter_to_img(const ReconFilterDev& f, const ImageSeg& seg, const floa
                         uint32_t channels, const float2* coords, uint32_t n, float multiplier,
                         float* pixels, float* counts, const ReconScratch& s, cudaStream_t stream) {
     if (n == 0 || seg.w <= 0 || seg.h <= 0) return 0;
-    return use_tiles(f) ? splat_tiles(f, seg, values, channels, coords, n, multiplier, pixels,
-                                      counts, s, stream)
-                        : splat_pairs(f, seg, values, channels, coords, n, multiplier, pixels,
-                                      counts, s, stream);
+    const auto splat = use_tiles(f, n, seg) ? splat_tiles : splat_pairs;
+    return splat(f, seg, values, channels, coords, n, multiplier, pixels, counts, s, stream);
 }
 
 int recon_filter_grid(const ReconFilterDev& f, const float4* samples, const float2* coords,

@@ -212,6 +212,20 @@ def test_splat_windows_at_image_edges(cuda, oracle, ftype, radius, params, chann
     assert _bits_equal(px, rp) and _bits_equal(cnt, rc)
 
 
+# either side of the line between tiles and pairs: 8 samples reaching a pixel
+# below 256 x 256 pixels, whatever their number from there on
+@pytest.mark.parametrize("w,h,per", [(40, 30, 7.9), (40, 30, 8.1), (256, 255, 8.1),
+                                     (256, 256, 8.1)])
+def test_splat_of_dense_samples(cuda, oracle, w, h, per):
+    rng = np.random.default_rng(w + h)
+    n = int(per * w * h / np.pi)  # radius 1
+    coords = np.stack([rng.uniform(0, w, n), rng.uniform(0, h, n)], 1).astype(np.float32)
+    values = rng.uniform(0, 4, (n, 4)).astype(np.float32)
+    px, cnt = _splat(cuda, "Tent", 1.0, {}, values, coords, (w, h))
+    rp, rc = oracle.filter_to_img("Tent", 1.0, values, coords, (w, h))
+    assert _bits_equal(px, rp) and _bits_equal(cnt, rc)
+
+
 def test_splat_of_crowded_pixels(cuda, oracle):
     """From none to hundreds of samples at a pixel; each pixel's sum is in the
     samples' order, so the bits are the oracle's."""
