@@ -38,6 +38,12 @@ constexpr uint32_t kSpinLimit = 1u << 24;
 struct PlocState {
     uint32_t m, base, steps;
 };
+// What the host reads after a batch: the last state, and the give-up word that
+// lies behind it (1 once a look-back has given up).
+struct PlocProgress {
+    PlocState state;
+    uint32_t gaveUp;
+};
 
 __device__ __forceinline__ void node_box(uint32_t g, const PlocIn& in, const float* inner,
                                          float b[6]) {
@@ -114,7 +120,9 @@ __device__ __forceinline__ void make_node(const PlocOut& out, uint32_t node, uin
 // 131 us in k_ploc_finish for the last kFinal clusters).
 // Counts and node numbers travel on the device: step k reads state k and
 // leaves state k + 1.  With kFinal clusters or fewer, or after a look-back that
-// gave up, a step does nothing.
+// gave up, a step does nothing.  The give-up word may be set while a block
+// starts, so one thread reads it for the block: the others' share of the boxes
+// is either there or not looked at.
 __global__ void __launch_bounds__(kStepBlock) k_ploc_step(const uint32_t* __restrict__ C,
                                                           uint32_t* __restrict__ Cout, PlocIn in,
                                                           PlocOut out, const PlocState* cur,
@@ -130,13 +138,14 @@ __global__ void __launch_bounds__(kStepBlock) k_ploc_step(const uint32_t* __rest
     const int tid = int(threadIdx.x);
     const PlocState st = *cur;
     const int m = int(st.m);
-    if (st.m <= uint32_t(kFinal) || *error) {
+    if (st.m <= uint32_t(kFinal)) {
         if (blockIdx.x == 0 && tid == 0) *next = st;
         return;
     }
-    if (tid == 0) tileId = atomicAdd(ticket, 1u);
+    if (tid == 0) tileId = *error ? kInvalid : atomicAdd(ticket, 1u);
     __syncthreads();
     const uint32_t tile = tileId;
+    if (tile == kInvalid) return;
     const int b0 = int(tile) * kTile;
     if (b0 >= m) return;
     for (int k = tid; k < kTile + 4 * kRadius; k += kStepBlock) {
@@ -278,10 +287,13 @@ __global__ void __launch_bounds__(kFinal) k_ploc_finish(const uint32_t* __restri
     }
 }
 
-__global__ void k_ploc_iota(uint32_t* C, uint32_t n, PlocState* state) {
+__global__ void k_ploc_iota(uint32_t* C, uint32_t n, PlocState* state, uint32_t* error) {
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
         C[i] = i;
-    if (blockIdx.x == 0 && threadIdx.x == 0) *state = PlocState{n, 0u, 0u};
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        *state = PlocState{n, 0u, 0u};
+        *error = 0u;
+    }
 }
 
 // Sum of the inner boxes' half surface areas (the SAH's node term) in
@@ -325,12 +337,13 @@ int inner_area_sum(const float* inner, uint32_t count, double* scratch8, double*
 namespace {
 size_t align256(size_t v) { return (v + 255) & ~size_t(255); }
 size_t step_tiles(uint32_t m) { return (size_t(m) + kTile - 1) / kTile; }
+constexpr size_t kStateBytes = kBatch * sizeof(PlocState) + sizeof(PlocProgress);
 }  // namespace
 
 size_t ploc_scratch_bytes(uint32_t n) {
-    // C x2; states and tickets; the tile status of a batch
-    return 2 * align256(size_t(n) * 4) + align256((kBatch + 1) * sizeof(PlocState)) +
-           align256((kBatch + 1) * 4) + align256(kBatch * step_tiles(n) * 8);
+    // C x2; the states; the tickets and the tile status of a batch
+    return 2 * align256(size_t(n) * 4) + align256(kStateBytes) + align256(kBatch * 4) +
+           align256(kBatch * step_tiles(n) * 8);
 }
 
 int ploc_build(const PlocIn& in, const PlocOut& out, void* scratch, uint32_t* iterations,
@@ -347,29 +360,36 @@ int ploc_build(const PlocIn& in, const PlocOut& out, void* scratch, uint32_t* it
         p += align256(size_t(n) * 4);
     }
     PlocState* state = reinterpret_cast<PlocState*>(p);
-    p += align256((kBatch + 1) * sizeof(PlocState));
-    uint32_t* tickets = reinterpret_cast<uint32_t*>(p);  // kBatch, then the error word
-    p += align256((kBatch + 1) * 4);
+    PlocProgress* progress = reinterpret_cast<PlocProgress*>(state + kBatch);
+    p += align256(kStateBytes);
+    uint32_t* tickets = reinterpret_cast<uint32_t*>(p);
+    p += align256(kBatch * 4);
     unsigned long long* status = reinterpret_cast<unsigned long long*>(p);
-    k_ploc_iota<<<grid_of(n, 256), 256, 0, st>>>(C[0], n, state);
+    k_ploc_iota<<<grid_of(n, 256), 256, 0, st>>>(C[0], n, state, &progress->gaveUp);
     MRB_CUDA(cudaGetLastError());
     PlocState h{n, 0u, 0u};
     // every step merges at least the pair with the globally least merged
     // area, so n - 1 steps bound the loop
     while (h.m > uint32_t(kFinal)) {
         const size_t tiles = step_tiles(h.m);
-        MRB_CUDA(cudaMemsetAsync(tickets, 0, align256((kBatch + 1) * 4) + kBatch * tiles * 8,
-                                 st));
+        MRB_CUDA(cudaMemsetAsync(tickets, 0, align256(kBatch * 4) + kBatch * tiles * 8, st));
         // an even number of steps: each batch starts from C[0]
         for (int k = 0; k < kBatch; k++)
             k_ploc_step<<<static_cast<uint32_t>(tiles), kStepBlock, 0, st>>>(
                 C[k & 1], C[(k & 1) ^ 1], in, out, state + k, state + k + 1, tickets + k,
-                tickets + kBatch, status + k * tiles);
+                &progress->gaveUp, status + k * tiles);
         MRB_CUDA(cudaGetLastError());
         const uint32_t before = h.m;
-        MRB_CUDA(cudaMemcpyAsync(&h, state + kBatch, sizeof(h), cudaMemcpyDeviceToHost, st));
-        MRB_CUDA(cudaMemcpyAsync(state, state + kBatch, sizeof(h), cudaMemcpyDeviceToDevice, st));
+        PlocProgress now;
+        MRB_CUDA(cudaMemcpyAsync(&now, progress, sizeof(now), cudaMemcpyDeviceToHost, st));
+        MRB_CUDA(cudaMemcpyAsync(state, &progress->state, sizeof(PlocState),
+                                 cudaMemcpyDeviceToDevice, st));
         MRB_CUDA(cudaStreamSynchronize(st));
+        if (now.gaveUp) {
+            set_error("PLOC: a look-back gave up");
+            return MRB_E_DEVICE;
+        }
+        h = now.state;
         if (h.m >= before || h.m + h.base != n) {
             set_error("PLOC: %u clusters and %u inner nodes of %u leaves after %u steps", h.m,
                       h.base, n, h.steps);
