@@ -340,10 +340,23 @@ size_t step_tiles(uint32_t m) { return (size_t(m) + kTile - 1) / kTile; }
 constexpr size_t kStateBytes = kBatch * sizeof(PlocState) + sizeof(PlocProgress);
 }  // namespace
 
-size_t ploc_scratch_bytes(uint32_t n) {
+PlocArrays ploc_arrays(uint32_t n) {
+    // in size_t throughout: the boxes alone pass 4 GB from 178,956,972 leaves on
+    const size_t inner = size_t(n) - 1;
+    PlocArrays a{};
+    auto take = [&](size_t bytes) {
+        const size_t at = a.bytes;
+        a.bytes += align256(bytes);
+        return at;
+    };
+    a.left = take(inner * 4);
+    a.right = take(inner * 4);
+    a.inner = take(inner * 24);
+    a.root = take(4);
     // C x2; the states; the tickets and the tile status of a batch
-    return 2 * align256(size_t(n) * 4) + align256(kStateBytes) + align256(kBatch * 4) +
-           align256(kBatch * step_tiles(n) * 8);
+    a.scratch = take(2 * align256(size_t(n) * 4) + align256(kStateBytes) + align256(kBatch * 4) +
+                     kBatch * step_tiles(n) * 8);
+    return a;
 }
 
 int ploc_build(const PlocIn& in, const PlocOut& out, void* scratch, uint32_t* iterations,

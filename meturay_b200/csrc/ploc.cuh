@@ -19,7 +19,12 @@ struct PlocOut {
     uint32_t* root;    // 1: global index of the root
 };
 
-size_t ploc_scratch_bytes(uint32_t n);
+// Byte offsets of a build's arrays (PlocOut's and the scratch) in one
+// allocation of `bytes`.
+struct PlocArrays {
+    size_t left, right, inner, root, scratch, bytes;
+};
+PlocArrays ploc_arrays(uint32_t n);
 // Sum of the half surface areas of `count` boxes (6 floats each); scratch8:
 // one device double.
 int inner_area_sum(const float* inner, uint32_t count, double* scratch8, double* out,

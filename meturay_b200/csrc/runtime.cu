@@ -1210,13 +1210,11 @@ int mrb_accel_construct(mrb_scene* s, void* stream) {
         // everything that lives only through the build comes out of one
         // allocation: the PLOC tree and its scratch, the collapse's, the probes'
         auto part = [](size_t bytes) { return (bytes + 255) & ~size_t(255); };
-        const size_t child = part((n - 1) * 4), boxes = part((n - 1) * 24);
         const size_t collapse = part(std::max(wide_scratch_bytes(n), wide_probe_bytes()));
         const bool ploc = s->wideTree != 0;
+        const PlocArrays pa = ploc_arrays(n);
         DBuf temp;
-        if ((r = temp.alloc(collapse +
-                            (ploc ? 2 * child + boxes + 256 + ploc_scratch_bytes(n) : 0))))
-            return r;
+        if ((r = temp.alloc(collapse + (ploc ? pa.bytes : 0)))) return r;
         char* tp = temp.as<char>() + collapse;
         WideBuildIn wi{n, s->aRoot.as<uint32_t>(), s->aLeft.as<uint32_t>(), s->aRight.as<uint32_t>(),
                        s->aInner.as<float>(), s->aTriAabb.as<float>(), s->aSorted.as<uint32_t>(),
@@ -1226,11 +1224,11 @@ int mrb_accel_construct(mrb_scene* s, void* stream) {
         // the Morton splits give the collapse better nodes to start from
         s->wideTreeUsed = 0;
         if (ploc) {
-            uint32_t* pLeft = reinterpret_cast<uint32_t*>(tp);
-            uint32_t* pRight = reinterpret_cast<uint32_t*>(tp + child);
-            float* pInner = reinterpret_cast<float*>(tp + 2 * child);
-            uint32_t* pRoot = reinterpret_cast<uint32_t*>(tp + 2 * child + boxes);
-            void* pScratch = tp + 2 * child + boxes + 256;
+            uint32_t* pLeft = reinterpret_cast<uint32_t*>(tp + pa.left);
+            uint32_t* pRight = reinterpret_cast<uint32_t*>(tp + pa.right);
+            float* pInner = reinterpret_cast<float*>(tp + pa.inner);
+            uint32_t* pRoot = reinterpret_cast<uint32_t*>(tp + pa.root);
+            void* pScratch = tp + pa.scratch;
             PlocIn pi{n, s->aTriAabb.as<float>(), s->aSorted.as<uint32_t>()};
             PlocOut po{pLeft, pRight, pInner, pRoot};
             if ((r = ploc_build(pi, po, pScratch, &s->plocSteps, st))) return r;

@@ -77,10 +77,27 @@ void give_up_while_a_block_starts() {
     }
 }
 
+// The arrays of a build neither overlap nor run out of the allocation, at
+// counts whose byte sizes pass 32 bits too.
+void arrays_of_large_builds() {
+    for (uint32_t n : {2u, 1000000u, 178956971u, 178956972u, 200000000u, 0x7FFFFFFFu}) {
+        const PlocArrays a = ploc_arrays(n);
+        const size_t inner = size_t(n) - 1;
+        const size_t at[6] = {a.left, a.right, a.inner, a.root, a.scratch, a.bytes};
+        const size_t need[5] = {4 * inner, 4 * inner, 24 * inner, 4, 8 * size_t(n)};
+        for (int i = 0; i < 5; i++)
+            expect(at[i] % 256 == 0 && at[i] + need[i] <= at[i + 1], "an array's room", int(n));
+    }
+}
+
 }  // namespace
 }  // namespace mrb
 
-int main() {
+int main(int, char** argv) {
+    if (!std::strcmp(argv[1], "arrays")) {
+        mrb::arrays_of_large_builds();
+        return mrb::failures ? 1 : 0;
+    }
     mrb::steps();
     mrb::give_up_while_a_block_starts();
     return mrb::failures ? 1 : 0;

@@ -29,6 +29,9 @@ def program(tmp_path_factory):
     return out
 
 
-def test_a_block_reads_the_give_up_word_once(program):
-    r = subprocess.run([str(program)], capture_output=True, text=True, timeout=120)
+@pytest.mark.parametrize("check", ["blocks", "arrays"])
+def test_on_the_host(program, check):
+    """blocks: a block acts on one reading of the give-up word; arrays: a build's
+    arrays have their room at any triangle count."""
+    r = subprocess.run([str(program), check], capture_output=True, text=True, timeout=120)
     assert r.returncode == 0, r.stdout + r.stderr
