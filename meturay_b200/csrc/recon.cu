@@ -7,17 +7,19 @@
 //   - the general entry point (any image coordinates) sorts a list with the
 //     onesweep sort, its length staying on the device (no host round trip, so
 //     the splat can sit inside a captured graph), and every pixel sums its
-//     samples in ascending sample order.  With a window of one or two pixels
-//     the list holds the pairs of pixel and sample (count, scan, write in sample
-//     order) and a thread sums a pixel's run; with larger ones it holds a
-//     sample once per tile of 8 x 8 pixels that its window touches, and a warp
-//     walks a tile's samples for half of its pixels;
+//     samples in ascending sample order.  With a radius below 0.75 the list
+//     holds the pairs of pixel and sample (count, scan, write in sample order)
+//     and a thread sums a pixel's run; with larger ones it holds a sample once
+//     per tile of 8 x 8 pixels that its window touches, and a warp walks a
+//     tile's samples for half of its pixels, or a block those of a tile on
+//     which samples crowd;
 //   - the tracer's own samples lie on the camera's stratified grid, so each
 //     pixel finds its candidates by index arithmetic in a small
 //     neighbourhood and sums them in the same ascending sample order: the
 //     same bits as the general path, with no pairs, no sort and no atomics.
 // Per pixel, ascending sample order is also the order of the reference's
 // own CPU expectation (Test_TracerCUDA/T_ReconFilter.cu:96-140).
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <type_traits>
@@ -81,7 +83,7 @@ __host__ __device__ inline bool in_segment(const ImageSeg& g, int32_t px, int32_
 }
 
 // ---------------------------------------------------------------------------
-// Windows of one or two pixels: pairs of pixel and sample
+// Small radii: pairs of pixel and sample
 // ---------------------------------------------------------------------------
 // Pass 1: number of (pixel, sample) pairs per sample.
 __global__ void __launch_bounds__(256) k_expand_count(const float2* __restrict__ coords, uint32_t n,
@@ -193,7 +195,7 @@ __global__ void __launch_bounds__(256) k_filter_pixels(
 }
 
 // ---------------------------------------------------------------------------
-// Larger windows: tiles of pixels
+// Larger radii: tiles of pixels
 // ---------------------------------------------------------------------------
 // Tiles of the segment that a sample's window touches.
 constexpr int32_t kTileSide = 8;
@@ -213,10 +215,14 @@ __device__ __forceinline__ TileSpan tile_span(const SamplePix& s, const ImageSeg
             int32_t(ay) / kTileSide, int32_t(by - 1) / kTileSide + 1};
 }
 
-// Pass 1: number of tiles per sample.
+// Pass 1: number of tiles per sample.  Also clears the tiles' runs and the
+// lengths of the lists behind them.
 __global__ void __launch_bounds__(256) k_tile_count(const float2* __restrict__ coords, uint32_t n,
                                                     uint32_t wh, ImageSeg g,
-                                                    uint32_t* __restrict__ count) {
+                                                    uint32_t* __restrict__ count,
+                                                    uint32_t* __restrict__ clear, uint32_t words) {
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < words; i += gridDim.x * blockDim.x)
+        clear[i] = 0u;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const float2 c = coords[i];
         const TileSpan t = tile_span(sample_pix(c.x, c.y, wh), g);
@@ -242,16 +248,201 @@ __global__ void __launch_bounds__(256) k_tile_write(const float2* __restrict__ c
     }
 }
 
+// A tile with more samples than this is taken by a block (crowded_tile) instead
+// of two warps.  Up to kFew tiles with over kCrowd samples lie on the SMs all at
+// once, and the longest walk of a warp is what the splat waits for; with more of
+// them the warps keep the SMs busy and a block gains only on long runs.  Radius 1,
+// whole splat, warps alone and blocks from 128 and 1,024 samples on (us): 20,000
+// samples in 10 x 10 pixels 651 and 164, in 100 x 100 (200 a tile) 68 and 60; but
+// 1080p (32,400 tiles) with 150 a tile 522 and 585 with blocks from 128 on.  640 x 360
+// (3,600 tiles) with 800 a tile 355 and 332 with blocks from 512 on, 1080p with 800
+// 2,450 and 2,600; 640 x 360 with 1,600 622 and 544.
+constexpr uint32_t kCrowd = 128, kDense = 1024, kFew = 1024;
+__device__ __forceinline__ uint32_t crowd_limit(uint32_t crowded) {
+    return crowded <= kFew ? kCrowd : kDense;
+}
+
 // Run boundaries of the sorted keys: [begin, end) for every tile that has
-// samples (both stay 0 for the others).
+// samples (both stay 0 for the others), and the lists of the tiles with long
+// runs: the sample kCrowd (kDense) places into a run enters its tile.  Past kFew
+// entries the first list is not used, so it need not be complete, and its
+// counter, which all of them would wait for, is left alone.
 __global__ void __launch_bounds__(256) k_tile_bounds(const uint32_t* __restrict__ keys,
                                                      const uint32_t* __restrict__ dCount,
-                                                     uint2* __restrict__ tiles) {
+                                                     uint2* __restrict__ tiles, CrowdLists lists) {
     const uint32_t n = *dCount;
+    auto enters = [&](uint32_t i, uint32_t k, uint32_t limit) {
+        return i >= limit && keys[i - limit] == k && (i == limit || keys[i - limit - 1] != k);
+    };
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const uint32_t k = keys[i];
         if (i == 0 || keys[i - 1] != k) tiles[k].x = i;
         if (i + 1 == n || keys[i + 1] != k) tiles[k].y = i + 1;
+        if (enters(i, k, kCrowd) && __ldcg(lists.counts) <= kFew)
+            lists.crowd[atomicAdd(lists.counts, 1u)] = k;
+        if (enters(i, k, kDense)) lists.dense[atomicAdd(lists.counts + 1, 1u)] = k;
+    }
+}
+
+// A pixel's sums into the image.
+template <int C>
+__device__ __forceinline__ void add_to_pixel(const ImageSeg& g, int32_t qx, int32_t qy,
+                                             const float* acc, float wsum,
+                                             float* __restrict__ pixels,
+                                             float* __restrict__ counts) {
+    const size_t q = size_t(qy) * size_t(g.w) + size_t(qx);
+    if constexpr (C == 4) {
+        float4* p4 = reinterpret_cast<float4*>(pixels) + q;
+        float4 p = *p4;
+        p.x += acc[0];
+        p.y += acc[1];
+        p.z += acc[2];
+        p.w += acc[3];
+        *p4 = p;
+    } else {
+        pixels[q] += acc[0];
+    }
+    counts[q] += wsum;
+}
+
+constexpr int kSplatBlock = 256;
+constexpr int kSplatWarps = kSplatBlock / 32;
+constexpr int kTilePixels = kTileSide * kTileSide;
+
+// A block's shared memory: samples (coordinates with the window's first pixel,
+// values) of each warp's round, or of a crowded tile's round with the votes.
+template <int C>
+struct SplatSmem {
+    typename std::conditional<C == 4, float4, float>::type value[kSplatBlock];
+    union {
+        float4 place[kSplatBlock];
+        struct {
+            float2 at[kSplatBlock];
+            uint32_t reach[kTilePixels][kSplatWarps + 1];       // a bit per sample of each warp
+            uint8_t list[kTilePixels][kSplatBlock + 4];         // a pixel's samples, ascending
+        } crowd;
+    };
+};
+
+// A tile with a long run, by a block: 256 samples a round, one per thread.  Each
+// warp votes, pixel by pixel, which of its 32 samples reach the pixel; four threads
+// per pixel make the votes a list and sum its samples in order, one channel each.
+// A warp of k_filter_tiles goes through a run 32 samples at a time and takes a step
+// for every sample that touches any of its 32 pixels; here eight warps share the
+// reads and tests, and a pixel's threads step over what does not reach it.  Bound
+// by the rounds' chain: some 1,200 cycles of votes, 900 of lists and 600 of sums.
+// Radius 1, whole splat, by pairs, by warps and so (us): 20,000 samples in one pixel
+// 2,505, 1,112 and 1,024; in 10 x 10 222, 651 and 164; in 30 x 30 100, 153 and 74;
+// 200,000 in 30 x 30 322, 1,024 and 239; 65,536 on 32 x 32 132, 324 and 99.  In 10 x 10 a
+// thread per pixel for all four channels took 192 and not 148 (both in a launch of
+// their own), the votes bit by bit instead of from a list 184 and not 163.
+template <int C>
+__device__ __forceinline__ void crowded_tile(SplatSmem<C>& S, uint2 range, int32_t ox, int32_t oy,
+                                             const uint32_t* __restrict__ vals,
+                                             const float* __restrict__ values,
+                                             const float2* __restrict__ coords,
+                                             const ReconFilterDev& f, const ImageSeg& g,
+                                             float multiplier, float* __restrict__ pixels,
+                                             float* __restrict__ counts) {
+    constexpr uint32_t kAll = 0xFFFFFFFFu;
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+    // four threads per pixel, one channel each
+    const uint32_t p = tid >> 2, part = tid & 3u;
+    const float r2 = f.radius * f.radius;
+    const int32_t qx = ox + int32_t(p & 7u), qy = oy + int32_t(p >> 3);
+    const float pcx = static_cast<float>(qx + g.offX) + 0.5f;
+    const float pcy = static_cast<float>(qy + g.offY) + 0.5f;
+    float acc = 0.0f, wsum = 0.0f;
+    bool hit = false;
+    // ids are read two rounds ahead, coordinates and values one
+    auto id_at = [&](uint32_t i) { return i < range.y ? __ldg(vals + i) : 0u; };
+    float2 c = make_float2(0.0f, 0.0f);
+    float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    auto sample_at = [&](uint32_t i, uint32_t id) {
+        if (i >= range.y) return;
+        c = __ldg(coords + id);
+        if constexpr (C == 4) v = __ldg(reinterpret_cast<const float4*>(values) + id);
+        else v.x = __ldg(values + id);
+    };
+    sample_at(range.x + tid, id_at(range.x + tid));
+    uint32_t id1 = id_at(range.x + kSplatBlock + tid);
+    for (uint32_t base = range.x; base < range.y; base += kSplatBlock) {
+        // squared distances to the tile's columns, infinite beyond the window
+        float dx2[kTileSide];
+        int32_t y0 = 0, y1 = 0;
+#pragma unroll
+        for (int k = 0; k < kTileSide; k++) dx2[k] = INFINITY;
+        if (base + tid < range.y) {
+            const SamplePix s = sample_pix(c.x, c.y, f.wh);
+            const int32_t x0 = s.ix + s.x0 - (ox + g.offX), x1 = x0 + (s.x1 - s.x0);
+            y0 = s.iy + s.y0 - (oy + g.offY);
+            y1 = y0 + (s.y1 - s.y0);
+#pragma unroll
+            for (int k = 0; k < kTileSide; k++) {
+                const float dx = c.x - (static_cast<float>(ox + g.offX + k) + 0.5f);
+                if (k >= x0 && k < x1) dx2[k] = dx * dx;
+            }
+        }
+#pragma unroll
+        for (int y = 0; y < kTileSide; y++) {
+            const float dy = c.y - (static_cast<float>(oy + g.offY + y) + 0.5f);
+            const float dy2 = (y >= y0 && y < y1) ? dy * dy : INFINITY;
+#pragma unroll
+            for (int x = 0; x < kTileSide; x++) {
+                const uint32_t reach = __ballot_sync(kAll, dx2[x] + dy2 <= r2);
+                if (lane == 0) S.crowd.reach[y * kTileSide + x][warp] = reach;
+            }
+        }
+        S.crowd.at[tid] = c;
+        if constexpr (C == 4) S.value[tid] = v;
+        else S.value[tid] = v.x;
+        const uint32_t i1 = base + kSplatBlock + tid;
+        sample_at(i1, id1);
+        id1 = id_at(i1 + kSplatBlock);
+        __syncthreads();
+        // the pixel's votes as a list, two words by each of its threads
+        uint32_t w0 = S.crowd.reach[p][2u * part], w1 = S.crowd.reach[p][2u * part + 1u];
+        const uint32_t own = uint32_t(__popc(w0) + __popc(w1));
+        uint32_t upTo = own;
+#pragma unroll
+        for (uint32_t o = 1; o < 4u; o <<= 1) {
+            const uint32_t below = __shfl_up_sync(kAll, upTo, o, 4);
+            if (part >= o) upTo += below;
+        }
+        const uint32_t count = __shfl_sync(kAll, upTo, 3, 4);
+        hit |= count > 0u;
+        uint8_t* out = S.crowd.list[p] + (upTo - own);
+        for (; w0; w0 &= w0 - 1u) *out++ = uint8_t(64u * part + uint32_t(__ffs(int(w0)) - 1));
+        for (; w1; w1 &= w1 - 1u)
+            *out++ = uint8_t(64u * part + 32u + uint32_t(__ffs(int(w1)) - 1));
+        __syncwarp();
+        // its samples in order, four at a time but for the sums
+        for (uint32_t k = 0; k < count; k += 4u) {
+            const uint32_t four = *reinterpret_cast<const uint32_t*>(&S.crowd.list[p][k]);
+            float weight[4], val[4];
+#pragma unroll
+            for (uint32_t j = 0; j < 4u; j++) {
+                const uint32_t h = (four >> (8u * j)) & 0xFFu;
+                const float2 at = S.crowd.at[h];
+                weight[j] = recon_weight(f, pcx, pcy, at.x, at.y) * multiplier;
+                if constexpr (C == 4)
+                    val[j] = reinterpret_cast<const float*>(&S.value[h])[part];
+                else
+                    val[j] = S.value[h];
+            }
+#pragma unroll
+            for (uint32_t j = 0; j < 4u; j++)
+                if (k + j < count) {
+                    wsum += weight[j];
+                    acc += weight[j] * val[j];
+                }
+        }
+        __syncthreads();
+    }
+    if (hit && qx < g.w && qy < g.h && in_segment(g, qx + g.offX, qy + g.offY)) {
+        const size_t q = size_t(qy) * size_t(g.w) + size_t(qx);
+        if (C == 4 || part == 0u) pixels[q * C + (C == 4 ? part : 0u)] += acc;
+        if (part == 0u) counts[q] += wsum;
     }
 }
 
@@ -260,32 +451,45 @@ __global__ void __launch_bounds__(256) k_tile_bounds(const uint32_t* __restrict_
 // keeps those whose window touches its pixels; then it takes these in order from
 // shared memory, every lane holding the sample against its own pixel.  So a pixel
 // sums its samples in ascending order, whatever their number.  Bound by the reads
-// of ids and coordinates, hence the two rounds ahead, and where samples crowd by
-// the steps of one warp per tile.  1M samples, 1080p, tent of radius 1, whole
-// splat: 341 us by pairs, 240 us so; 20,000 samples in one pixel: 2,500 us and 1,120.
-// Tiles of 16 x 16 (1.3 entries per sample instead of 1.6): 250 us and 2,770.
+// of ids and coordinates, hence the two rounds ahead.  1M samples, 1080p, tent of
+// radius 1, whole splat: 340 us by pairs, 228 us so.  Tiles of 16 x 16 (1.3 entries
+// per sample instead of 1.6) were 4 % slower.
+// The last crowdBlocks blocks take the crowded tiles.  In a launch of their own
+// these cost 4 us a call and start only after the others; six blocks per SM (40
+// registers) because at five the reads of sparse images are slower (100,000 samples
+// on 1080p 90 and 94 us), although crowds gain 8 %.
 template <int C, int kType>
-__global__ void __launch_bounds__(256) k_filter_tiles(
-    const uint2* __restrict__ tiles, int32_t tilesX, const uint32_t* __restrict__ vals,
-    const float* __restrict__ values, const float2* __restrict__ coords, ReconFilterDev f,
-    ImageSeg g, float multiplier, float* __restrict__ pixels, float* __restrict__ counts) {
+__global__ void __launch_bounds__(kSplatBlock, 6) k_filter_tiles(
+    const uint2* __restrict__ tiles, CrowdLists lists, uint32_t crowdBlocks, int32_t tilesX,
+    const uint32_t* __restrict__ vals, const float* __restrict__ values,
+    const float2* __restrict__ coords, ReconFilterDev f, ImageSeg g, float multiplier,
+    float* __restrict__ pixels, float* __restrict__ counts) {
     constexpr uint32_t kAll = 0xFFFFFFFFu;
-    __shared__ float4 place[8][32];  // coordinates, the window's first pixel
-    __shared__ __align__(16) float value[8][32][C];
+    __shared__ __align__(16) SplatSmem<C> S;
+    f.type = kType;
+    if (blockIdx.x >= gridDim.x - crowdBlocks) {
+        const bool few = lists.counts[0] <= kFew;
+        const uint32_t count = lists.counts[few ? 0 : 1];
+        for (uint32_t i = blockIdx.x - (gridDim.x - crowdBlocks); i < count; i += crowdBlocks) {
+            const int32_t t = int32_t((few ? lists.crowd : lists.dense)[i]);
+            crowded_tile<C>(S, tiles[t], (t % tilesX) * kTileSide, (t / tilesX) * kTileSide, vals,
+                            values, coords, f, g, multiplier, pixels, counts);
+        }
+        return;
+    }
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     // the warp's and the lane's pixel, in the segment
-    const int32_t blocksX = (tilesX + 1) / 2;
-    const int32_t wx = (int32_t(blockIdx.x) % blocksX) * 16 + int32_t(warp & 1u) * 8;
-    const int32_t wy = (int32_t(blockIdx.x) / blocksX) * 16 + int32_t(warp >> 1) * 4;
+    const int32_t blocksX = (tilesX + 1) / 2, block = int32_t(blockIdx.x);
+    const int32_t wx = (block % blocksX) * 16 + int32_t(warp & 1u) * 8;
+    const int32_t wy = (block / blocksX) * 16 + int32_t(warp >> 1) * 4;
     if (wx >= g.w || wy >= g.h) return;
     const uint2 range = tiles[(wy / kTileSide) * tilesX + wx / kTileSide];
-    if (range.x == range.y) return;
-    f.type = kType;
+    if (range.x == range.y || range.y - range.x > crowd_limit(lists.counts[0])) return;
+    const uint32_t mine = 32u * warp;  // this warp's place in S
     const int32_t qx = wx + int32_t(lane & 7u), qy = wy + int32_t(lane >> 3);
     const int32_t gx = qx + g.offX, gy = qy + g.offY;
     const float pcx = static_cast<float>(gx) + 0.5f, pcy = static_cast<float>(gy) + 0.5f;
-    // a window of one pixel reaches it wherever the sample lies in it
-    const float r2 = f.wh == 1u ? INFINITY : f.radius * f.radius;
+    const float r2 = f.radius * f.radius;
     const SamplePix any = sample_pix(0.5f, 0.5f, f.wh);
     const int32_t extent = any.x1 - any.x0;  // of a window, per axis
     float acc[C];
@@ -315,18 +519,18 @@ __global__ void __launch_bounds__(256) k_filter_tiles(
         const uint32_t some = __ballot_sync(kAll, touches);
         if (touches) {
             const uint32_t at = uint32_t(__popc(some & ((1u << lane) - 1u)));
-            place[warp][at] = make_float4(c.x, c.y, __int_as_float(lowX), __int_as_float(lowY));
+            S.place[mine + at] = make_float4(c.x, c.y, __int_as_float(lowX), __int_as_float(lowY));
             if constexpr (C == 4)
-                *reinterpret_cast<float4*>(value[warp][at]) =
-                    reinterpret_cast<const float4*>(values)[id];
+                S.value[mine + at] = reinterpret_cast<const float4*>(values)[id];
             else
-                value[warp][at][0] = values[id];
+                S.value[mine + at] = values[id];
         }
         __syncwarp();
         const int count = __popc(some);
 #pragma unroll 4
         for (int h = 0; h < count; h++) {
-            const float4 s = place[warp][h];
+            const float4 s = S.place[mine + uint32_t(h)];
+            const float* v = reinterpret_cast<const float*>(&S.value[mine + uint32_t(h)]);
             const float dx = s.x - pcx, dy = s.y - pcy;
             const bool reaches =
                 (uint32_t(gx - __float_as_int(s.z)) < uint32_t(extent)) &
@@ -336,7 +540,7 @@ __global__ void __launch_bounds__(256) k_filter_tiles(
             if (kType <= kReconTent || reaches) w = recon_weight(f, pcx, pcy, s.x, s.y) * multiplier;
             wsum = reaches ? wsum + w : wsum;
             for (int k = 0; k < C; k++)
-                acc[k] = reaches ? acc[k] + w * value[warp][h][k] : acc[k];
+                acc[k] = reaches ? acc[k] + w * v[k] : acc[k];
             hit |= reaches;
         }
         __syncwarp();
@@ -345,20 +549,8 @@ __global__ void __launch_bounds__(256) k_filter_tiles(
         c = c1;
     }
     // a tile may stick out of the segment and a segment out of the image
-    if (!hit || qx >= g.w || qy >= g.h || !in_segment(g, gx, gy)) return;
-    const size_t q = size_t(qy) * size_t(g.w) + size_t(qx);
-    if constexpr (C == 4) {
-        float4* p4 = reinterpret_cast<float4*>(pixels) + q;
-        float4 p = *p4;
-        p.x += acc[0];
-        p.y += acc[1];
-        p.z += acc[2];
-        p.w += acc[3];
-        *p4 = p;
-    } else {
-        pixels[q] += acc[0];
-    }
-    counts[q] += wsum;
+    if (hit && qx < g.w && qy < g.h && in_segment(g, gx, gy))
+        add_to_pixel<C>(g, qx, qy, acc, wsum, pixels, counts);
 }
 
 // Tracer splat over the camera's sample grid.  Sample sid = sy * (W*sp) + sx
@@ -600,19 +792,12 @@ static uint32_t tile_total(const ImageSeg& seg) {
 }
 
 // Whether a splat lists samples by tile or by pixel.  A sample reaches pi r^2
-// pixels and touches (1 + (wh - 1) / 8)^2 tiles on average: 3.1 and 1.6 with a
-// radius of 1 (a window of 3), 0.8 and 1.3 with 0.5 (of 2).  Radius 1, 1M samples
-// on 1080p: by tiles 233 us, by pairs 343; radius 0.5, 2.6M samples: 410 and 304.
-// Where many samples crowd on few tiles (over kDense reaching a pixel of an image
-// below kWide pixels) their warps' serial walks take longer than the sort of the
-// pairs: radius 1.33, 154,930 samples on 79 x 72 214 us and 182, radius 0.75, 16
-// reaching a pixel of 256 x 256 169 and 151; 16 with a radius of 1 112 and 145.
-static bool use_tiles(const ReconFilterDev& f, uint32_t n, const ImageSeg& seg) {
-    constexpr double kDense = 8.0, kWide = 65536.0;
-    const double pix = double(seg.w) * double(seg.h);
-    const bool dense = double(n) * 3.1416 * double(f.radius) * double(f.radius) > kDense * pix;
-    return f.wh >= 3u && (!dense || (pix >= kWide && f.radius >= 1.0f));
-}
+// pixels and touches (1 + (wh - 1) / 8)^2 tiles on average: 1.8 and 1.6 with a radius
+// of 0.75, 1.1 and 1.6 with 0.6.  Pairs and tiles, whole splat (us), 104,000 and 4.1M
+// samples on 1080p, then 16,000 on 128 x 128 and 262,000 on 256 x 256: radius 0.6 94 and 90,
+// 515 and 681, 58 and 55, 81 and 101; 0.75 98 and 90, 677 and 689, 58 and 54, 89 and 90;
+// 0.8 102 and 90, 753 and 691, 59 and 54, 92 and 91.
+static bool use_tiles(const ReconFilterDev& f) { return f.radius >= 0.75f; }
 
 // Carves the scratch of a splat out of base (null: only adds up its bytes).
 static size_t carve(unsigned char* base, const ReconFilterDev& f, uint32_t n, const ImageSeg& seg,
@@ -623,7 +808,7 @@ static size_t carve(unsigned char* base, const ReconFilterDev& f, uint32_t n, co
         at += align256(bytes);
         return p;
     };
-    const bool tiles = use_tiles(f, n, seg);
+    const bool tiles = use_tiles(f);
     const size_t entries = size_t(n) * (tiles ? tiles_per_sample(f) : f.wh * f.wh);
     const size_t lists = tiles ? tile_total(seg) : size_t(seg.w) * size_t(seg.h);
     s.count = reinterpret_cast<uint32_t*>(take((size_t(n) + 1) * 4));
@@ -636,7 +821,15 @@ static size_t carve(unsigned char* base, const ReconFilterDev& f, uint32_t n, co
     s.sortTempBytes = radix_sort_temp_bytes(s.entries, 4, 0, s.bits);
     s.sortTemp = take(s.sortTempBytes);
     if (tiles) {
-        s.tiles = reinterpret_cast<uint2*>(take(lists * 8));
+        // runs, the number of crowded tiles (cleared with them) and their list
+        // the runs, the lengths of the two lists (cleared with them), the lists: a
+        // tile in one has more than kCrowd (kDense) entries
+        const size_t crowd = std::min(lists, entries / kCrowd);
+        s.tiles = reinterpret_cast<uint2*>(
+            take(lists * 8 + 8 + (crowd + std::min(lists, entries / kDense)) * 4));
+        s.crowds.counts = reinterpret_cast<uint32_t*>(s.tiles + lists);
+        s.crowds.crowd = s.crowds.counts + 2;
+        s.crowds.dense = s.crowds.crowd + crowd;
     } else {
         s.begin = reinterpret_cast<uint32_t*>(take(lists * 4));
         s.end = reinterpret_cast<uint32_t*>(take(lists * 4));
@@ -687,19 +880,26 @@ static int splat_tiles(const ReconFilterDev& f, const ImageSeg& seg, const float
                        float* pixels, float* counts, const ReconScratch& s, cudaStream_t stream) {
     const int32_t columns = static_cast<int32_t>(tile_columns(seg));
     const uint32_t g = grid_of(n, 148 * 8);
-    k_tile_count<<<g, 256, 0, stream>>>(coords, n, f.wh, seg, s.count);
+    const uint32_t words = 2u * tile_total(seg) + 2u;
+    k_tile_count<<<grid_of(std::max(n, words), 148 * 8), 256, 0, stream>>>(
+        coords, n, f.wh, seg, s.count, reinterpret_cast<uint32_t*>(s.tiles), words);
     if (exclusive_scan_u32(s.count, s.offset, n, s.scanTemp, stream)) return MRB_E_CUDA;
     k_tile_write<<<g, 256, 0, stream>>>(coords, n, f.wh, seg, columns, s.offset, s.keys, s.vals);
     const uint32_t* dTotal = s.offset + n;
     if (radix_sort_pairs<uint32_t>(s.keys, s.vals, dTotal, s.entries, 0, s.bits, false, s.sortTemp,
                                    s.sortTempBytes, stream, false))
         return MRB_E_CUDA;
-    MRB_CUDA(cudaMemsetAsync(s.tiles, 0, size_t(tile_total(seg)) * 8, stream));
-    k_tile_bounds<<<grid_of(s.entries, 148 * 8), 256, 0, stream>>>(s.keys, dTotal, s.tiles);
-    const uint32_t blocks = (uint32_t(seg.w - 1) / 16u + 1u) * (uint32_t(seg.h - 1) / 16u + 1u);
+    k_tile_bounds<<<grid_of(s.entries, 148 * 8), 256, 0, stream>>>(s.keys, dTotal, s.tiles,
+                                                                   s.crowds);
+    // a tile lists a sample once, so few samples crowd no tile
+    const uint32_t crowdBlocks =
+        n > kCrowd ? std::min({148u * 6u, tile_total(seg), s.entries / kCrowd}) : 0u;
+    const uint32_t blocks =
+        crowdBlocks + (uint32_t(seg.w - 1) / 16u + 1u) * (uint32_t(seg.h - 1) / 16u + 1u);
     auto launch = [&](auto ch, auto type) {
-        k_filter_tiles<decltype(ch)::value, decltype(type)::value><<<blocks, 256, 0, stream>>>(
-            s.tiles, columns, s.vals, values, coords, f, seg, multiplier, pixels, counts);
+        k_filter_tiles<decltype(ch)::value, decltype(type)::value>
+            <<<blocks, kSplatBlock, 0, stream>>>(s.tiles, s.crowds, crowdBlocks, columns, s.vals,
+                                                 values, coords, f, seg, multiplier, pixels, counts);
     };
     auto of_type = [&](auto ch) {
         switch (f.type) {
@@ -719,7 +919,7 @@ int recon_filter_to_img(const ReconFilterDev& f, const ImageSeg& seg, const floa
                         uint32_t channels, const float2* coords, uint32_t n, float multiplier,
                         float* pixels, float* counts, const ReconScratch& s, cudaStream_t stream) {
     if (n == 0 || seg.w <= 0 || seg.h <= 0) return 0;
-    const auto splat = use_tiles(f, n, seg) ? splat_tiles : splat_pairs;
+    const auto splat = use_tiles(f) ? splat_tiles : splat_pairs;
     return splat(f, seg, values, channels, coords, n, multiplier, pixels, counts, s, stream);
 }
 

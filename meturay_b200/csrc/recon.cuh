@@ -90,6 +90,12 @@ struct ImageSeg {
 int recon_filter_make(const char* type, float radius, uint32_t optCount, const char* const* names,
                       const float* values, ReconFilterDev* out);
 
+// Tiles with long runs of samples, by two lengths of run.
+struct CrowdLists {
+    uint32_t* counts;  // of tiles in crowd, of tiles in dense
+    uint32_t *crowd, *dense;
+};
+
 // General splat of arbitrary (value, image coordinate) samples: the
 // expand -> sort -> per-pixel reduction of FilterToImgInternal.
 // channels: 1 (float values, R image) or 4 (float4 values, RGBA image).
@@ -106,6 +112,7 @@ struct ReconScratch {
     uint32_t* begin;      // segment pixels (pairs)
     uint32_t* end;        // segment pixels (pairs)
     uint2* tiles;         // per tile of the segment: its run [x, y)
+    CrowdLists crowds;    // tiles: those with long runs
 };
 size_t recon_scratch_bytes(const ReconFilterDev& f, uint32_t n, const ImageSeg& seg);
 ReconScratch recon_scratch_carve(void* base, const ReconFilterDev& f, uint32_t n,

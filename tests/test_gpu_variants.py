@@ -193,15 +193,42 @@ def _splat(torch, ftype, radius, params, values, coords, res, segment=None):
     return img.get_image()
 
 
-# windows of 1 and 2 pixels (pairs), of 3 to 5 (tiles), and one wider than a tile of the sorted lists
+def _longest_run(radius, coords, segment):
+    """The most samples whose window touches one tile of 8 x 8 pixels."""
+    import meturay_b200 as m
+    wh = m.filter_pixel_wh(radius)
+    ox, oy, w, h = segment
+    c = coords[(np.abs(coords) < 1e9).all(1)]
+    i = np.trunc(c).astype(np.int64)
+    lo = i - (wh - 1) // 2 - ((wh % 2 == 0) & (c - i < 0.5)) - [ox, oy]
+    hi = lo + wh
+    lo, hi = np.maximum(lo, 0), np.minimum(hi, [w, h])
+    keep = (lo < hi).all(1)
+    a, b = lo[keep] // 8, (hi[keep] - 1) // 8
+    runs = np.zeros(((h + 7) // 8 + 1, (w + 7) // 8 + 1), np.int64)  # as a 2D difference
+    for x, y, v in ((a[:, 0], a[:, 1], 1), (b[:, 0] + 1, a[:, 1], -1), (a[:, 0], b[:, 1] + 1, -1),
+                    (b[:, 0] + 1, b[:, 1] + 1, 1)):
+        np.add.at(runs, (y, x), v)
+    return int(runs.cumsum(0).cumsum(1).max())
+
+
+CROWD = 128  # samples on a tile beyond which a block takes it and not two warps
+
+
+# Radii below 0.75 go by pairs of pixel and sample, from there on by tiles of
+# 8 x 8 pixels; windows of 1 to 5 pixels and one wider than a tile.  The numbers of
+# samples give tiles of less than a warp's round, of several, and of one and several
+# rounds of a block.
 @pytest.mark.parametrize("ftype,radius,params", [
-    ("Box", 0.0, {}), ("Box", 0.25, {}), ("Box", 0.5, {}), ("Tent", 0.75, {}), ("Tent", 1.0, {}),
-    ("Gaussian", 1.25, {"alpha": 1.0}), ("Mitchell", 2.0, {"b": 1 / 3, "c": 1 / 3}),
-    ("Tent", 9.25, {})])
+    ("Box", 0.0, {}), ("Box", 0.25, {}), ("Box", 0.5, {}), ("Tent", 0.74, {}), ("Tent", 0.75, {}),
+    ("Tent", 1.0, {}), ("Box", 1.25, {}), ("Gaussian", 1.25, {"alpha": 1.0}),
+    ("Mitchell", 2.0, {"b": 1 / 3, "c": 1 / 3}), ("Tent", 9.25, {})])
 @pytest.mark.parametrize("channels", [1, 4])
-def test_splat_windows_at_image_edges(cuda, oracle, ftype, radius, params, channels):
+@pytest.mark.parametrize("n", [300, 2000, 9000, 60_000])
+def test_splat_windows_at_image_edges(cuda, oracle, ftype, radius, params, channels, n):
+    import meturay_b200 as m
     rng = np.random.default_rng(int(radius * 100) + channels)
-    n, w, h = 9000, 67, 41
+    w, h = 67, 41
     coords = np.stack([rng.uniform(-4, w + 4, n), rng.uniform(-4, h + 4, n)], 1).astype(np.float32)
     coords[:6] = [[0, 0], [w, h], [np.nan, 3], [3, np.inf], [2e9, 1], [-0.5, -0.5]]
     values = rng.uniform(0, 8, (n, channels)).astype(np.float32)
@@ -210,12 +237,24 @@ def test_splat_windows_at_image_edges(cuda, oracle, ftype, radius, params, chann
     px, cnt = _splat(cuda, ftype, radius, params, values, coords, (w, h), seg)
     rp, rc = oracle.filter_to_img(ftype, radius, values, coords, (w, h), segment=seg, **params)
     assert _bits_equal(px, rp) and _bits_equal(cnt, rc)
+    # the route that this case stands for: pairs and their sort's second copy fill
+    # 16 bytes for each pixel of a window, tiles far less
+    flt = m.ReconFilter(ftype, radius, params)
+    img = m.ImageMemory(w, h, channels)
+    img.reportion(seg[:2], (seg[0] + seg[2], seg[1] + seg[3]))
+    flt.filter_to_img(img, _dev(cuda, values), _dev(cuda, coords), n)
+    cuda.cuda.synchronize()
+    if n >= 2000:
+        assert (flt.used_gpu_memory() > 16 * n * m.filter_pixel_wh(radius) ** 2) == (radius < 0.75)
+    if radius >= 0.75:
+        blocks = n >= 9000 or (n >= 2000 and radius > 9.0)
+        assert (_longest_run(radius, coords, seg) > CROWD) == blocks
 
 
-# either side of the line between tiles and pairs: 8 samples reaching a pixel
-# below 256 x 256 pixels, whatever their number from there on
+# few and many crowded tiles (1,024 is the line), the many with and without runs
+# that a block takes all the same (over 1,024 samples)
 @pytest.mark.parametrize("w,h,per", [(40, 30, 7.9), (40, 30, 8.1), (256, 255, 8.1),
-                                     (256, 256, 8.1)])
+                                     (256, 256, 8.1), (280, 280, 8.1), (280, 280, 40.0)])
 def test_splat_of_dense_samples(cuda, oracle, w, h, per):
     rng = np.random.default_rng(w + h)
     n = int(per * w * h / np.pi)  # radius 1
@@ -240,6 +279,36 @@ def test_splat_of_crowded_pixels(cuda, oracle):
         px, cnt = _splat(cuda, ftype, radius, params, values, coords, (w, h))
         rp, rc = oracle.filter_to_img(ftype, radius, values, coords, (w, h), **params)
         assert _bits_equal(px, rp) and _bits_equal(cnt, rc)
+
+
+def _splat_us(torch, coords, values, radius, res):
+    """Microseconds of a splat, the best of some on the device."""
+    import meturay_b200 as m
+    img, flt = m.ImageMemory(res[0], res[1], 4), m.ReconFilter("Tent", radius)
+    c, v = _dev(torch, coords), _dev(torch, values)
+    best = float("inf")
+    for _ in range(12):
+        a, b = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+        a.record()
+        for _ in range(4):
+            flt.filter_to_img(img, v, c, len(coords))
+        b.record()
+        torch.cuda.synchronize()
+        best = min(best, a.elapsed_time(b) * 250.0)
+    return best
+
+
+def test_crowded_samples_cost_little_more_than_spread_ones(cuda):
+    """200,000 samples on 30 x 30 pixels of a large image and all over it.  With a
+    pair per pixel that a sample reaches the first took 2 to 2.5 times the second,
+    and 8 times with one warp for every 8 x 4 pixels."""
+    rng = np.random.default_rng(4)
+    n, w, h = 200_000, 1920, 1080
+    spread = rng.uniform(0, 1, (n, 2)).astype(np.float32)
+    values = rng.uniform(0, 1, (n, 4)).astype(np.float32)
+    few = _splat_us(cuda, spread * np.float32([w, h]), values, 1.0, (w, h))
+    crowd = _splat_us(cuda, spread * np.float32(30.0) + np.float32([900, 500]), values, 1.0, (w, h))
+    assert crowd < 4.0 * few, (crowd, few)
 
 
 # ---- shadow rays -------------------------------------------------------------
