@@ -156,8 +156,8 @@ int mrb_accel_info(const mrb_scene* scene, uint32_t* info4);
  * mrb_tracer_render_frame runs before it captures its graph traces every
  * depth's rays with every kernel and keeps the fastest per depth (once per
  * tracer and traversal setting); mrb_accel_hit traces up to 32,768 rays with
- * a warp each.  Closest hits are the same with every kernel, up to the choice
- * among triangles at the same distance. */
+ * a warp each, fewer over small scenes.  Closest hits are the same with every
+ * kernel, up to the choice among triangles at the same distance. */
 #define MRB_WIDE_SORTED 0
 #define MRB_WIDE_OCTANT 1
 #define MRB_WIDE_SORTED_REFILL 2

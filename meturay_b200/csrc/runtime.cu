@@ -1343,7 +1343,8 @@ int mrb_accel_hit(const mrb_scene* s, const float* rayO, const float* rayD, uint
         MRB_CUDA(cudaMemset(flag.p, 0, 16));
     }
     // few rays: a warp each, unless a kernel was asked for by name
-    if (s->traversal == 1 && s->T > 1 && s->wideOrderMode == MRB_WIDE_AUTO && n <= kWideWarpRays)
+    if (s->traversal == 1 && s->T > 1 && s->wideOrderMode == MRB_WIDE_AUTO &&
+        n <= wide_warp_rays(s->T))
         return trace_closest_wide_few(s->wide(), reinterpret_cast<const float4*>(rayO),
                                       reinterpret_cast<const float4*>(rayD), n, ho,
                                       flag.as<uint32_t>(), static_cast<cudaStream_t>(stream));

@@ -947,9 +947,9 @@ __global__ void __launch_bounds__(128, 8) k_trace_wide_refill(WideAccelDev acc,
 // first.  Entries keep their distance and are dropped once a nearer hit is
 // known.  The nodes taken beside the top one are speculative; what they cost
 // is idle hardware here, which is why larger launches trace with one lane per
-// ray.  The fastest of those kernels and this one, clusters 1M and Cornell: 2,000
-// rays 97 and 24 us, 41 and 13; 16,000 rays 103 and 60, 58 and 27; 32,000 rays 110
-// and 102, 60 and 46; the same at 64,000 (hence kWideWarpRays).
+// ray (wide_warp_rays).  The fastest of those kernels and this one, random rays over
+// clusters 1M and Cornell: 2,000 rays 97 and 24 us, 41 and 13; 16,000 rays 103 and
+// 60, 58 and 27; 32,000 rays 110 and 102, 60 and 46; the same at 64,000.
 constexpr int kWarpStack = 256;       // entries per warp
 constexpr int kWarpBlock = 128;
 

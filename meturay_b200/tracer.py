@@ -176,7 +176,8 @@ class GPUScene:
         "sorted_refill", "octant_refill" (or 0-3), or "auto" (4, default):
         the fastest, timed on seeded probe rays at construction and then per
         depth on a tracer's own rays in the frame before it captures its
-        graph; `hit` traces up to 32,768 rays with a warp each."""
+        graph; `hit` traces up to 32,768 rays with a warp each, fewer over
+        small scenes."""
         if isinstance(order, str):
             order = WIDE_AUTO if order == "auto" else WIDE_ORDERS.index(order)
         check(lib.mrb_accel_set_wide_order(self._h, int(order)))

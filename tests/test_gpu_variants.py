@@ -343,15 +343,22 @@ def test_shadow_rays_see_what_the_binary_traversal_sees(system, cuda, order, shi
 
 
 # ---- few rays ----------------------------------------------------------------
-@pytest.mark.parametrize("name", ["clusters", "cornell"])
-@pytest.mark.parametrize("n", [1, 3, 4, 5, 2000, 32767, 32768, 32769])
+# the lines are at 4,096 rays below 64 triangles, 8,192 below 256, 16,384 below
+# 4,096, and 32,768
+@pytest.mark.parametrize("name,n", [
+    *((s, n) for s in ("clusters", "cornell") for n in (1, 3, 4, 5, 2000, 32767, 32768, 32769)),
+    *((s, n) for s in (2, 63) for n in (1, 4096, 4097)), (64, 8192), (255, 8193), (256, 16384),
+    (4095, 16385), (4096, 32768)])
 def test_few_rays_hit_what_a_lane_per_ray_hits(system, cuda, name, n):
-    """Up to 32,768 rays a warp traces each ray, with the same triangle test:
-    the distances are the same bits, and the triangles too but for ties."""
+    """Up to 32,768 rays, fewer over small scenes, a warp traces each ray, with the
+    same triangle test: the distances are the same bits, and the triangles too but
+    for ties."""
     import meturay_b200 as m
     torch = cuda
-    scene = m.scenes.clusters(1, n_clusters=40) if name == "clusters" else m.scenes.cornell(seed=1)
-    size = 100.0 if name == "clusters" else 1.0
+    scene = (m.scenes.clusters(1, n_clusters=40) if name == "clusters" else
+             m.scenes.cornell(seed=1) if name == "cornell" else
+             m.scenes.random_triangles(name, name))
+    size = 100.0 if name == "clusters" else 1.0 if name == "cornell" else 10.0
     g = m.GPUScene(system, scene)
     g.construct_accelerators()
     gen = torch.Generator(device="cuda").manual_seed(n)
@@ -378,3 +385,35 @@ def test_few_rays_hit_what_a_lane_per_ray_hits(system, cuda, name, n):
     assert int((~same).sum()) <= 1 + n // 1000
     assert torch.equal(few[0][same], lanes[0][same])
     assert torch.equal(few[3][same], lanes[3][same])
+
+
+@pytest.mark.parametrize("triangles,n", [(12, 32768), (100, 32768), (300, 32768)])
+def test_many_rays_over_a_small_scene_cost_no_more_than_a_lane_each(system, cuda, triangles, n):
+    """A warp per ray took 1.5 to 2.4 times the fastest form of a lane per ray here."""
+    import meturay_b200 as m
+    torch = cuda
+    g = m.GPUScene(system, m.scenes.random_triangles(triangles, triangles))
+    g.construct_accelerators()
+    gen = torch.Generator(device="cuda").manual_seed(n)
+    o = torch.rand((n, 4), generator=gen, device="cuda") * 10.0
+    d = torch.randn((n, 4), generator=gen, device="cuda")
+    d[:, :3] /= d[:, :3].norm(dim=1, keepdim=True)
+    o[:, 3], d[:, 3] = 0.0, 1000.0
+    out = [torch.zeros(n, dtype=torch.int32, device="cuda") for _ in range(2)]
+    out += [torch.zeros(n, device="cuda"), torch.zeros((n, 2), device="cuda")]
+
+    def micros(order):
+        g.set_wide_order(order)
+        best = float("inf")
+        for _ in range(12):
+            a, b = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            a.record()
+            for _ in range(20):
+                g.hit(o.data_ptr(), d.data_ptr(), n, *(x.data_ptr() for x in out))
+            b.record()
+            torch.cuda.synchronize()
+            best = min(best, a.elapsed_time(b) * 50.0)
+        return best
+
+    auto, lanes = micros("auto"), min(micros("sorted"), micros("octant"))
+    assert auto < 1.3 * lanes, (auto, lanes)
