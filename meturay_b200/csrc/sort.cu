@@ -44,12 +44,13 @@ constexpr int kItems = 16;
 constexpr int kTile = kThreads * kItems;  // 4096
 // Up to kSmallCount elements the tiles are of 1,024, up to kMidCount of 2,048:
 // the block's serial part (the ranking, item by item) is shorter and more SMs
-// work, while the look-back has more tiles to walk.  Three passes of 32-bit pairs
-// with kTile and with these tiles: 65,536 pairs 65 and 43 us, 300,000 73 and 57,
-// 600,000 80 and 67; at 1,000,000 both take 99.
+// work, while the look-back has more tiles to walk.  Three passes of 32-bit pairs,
+// then eight of 64-bit Morton codes, with these tiles and with kTile (us): 65,536
+// pairs 43 and 65; 300,000 58 and 65, 117 and 133; 400,000 67 and 63, 134 and 134;
+// 450,000 72 and 65, 134 and 134; 600,000 73 and 72, 150 and 149.
 constexpr int kSmallItems = 4, kMidItems = 8;
 constexpr uint32_t kSmallCount = 200u * kThreads * kSmallItems;
-constexpr uint32_t kMidCount = 320u * kThreads * kMidItems;
+constexpr uint32_t kMidCount = 200u * kThreads * kMidItems;
 __host__ __device__ __forceinline__ uint32_t tile_size(uint32_t n) {
     return uint32_t(kThreads) * (n <= kSmallCount ? kSmallItems : n <= kMidCount ? kMidItems : kItems);
 }
@@ -198,18 +199,31 @@ __device__ __forceinline__ void block_exclusive2(uint32_t a, uint32_t b, uint32_
 // One pass.  Blocks take tiles by ticket until none is left; hist holds the
 // pass's digit counts, scanned here.  kDense: keysIn are HitKeys.  keysOut
 // may be null (the last pass of a caller that only wants the order).
-// Four blocks per SM (three with 8-byte keys): digit and rank share a register
-// and the values are read when they are needed, at 128 registers two blocks ran.
-template <class K>
-constexpr int kSweepBlocks = sizeof(K) == 8 ? 3 : 4;
+// Two blocks per SM (128 registers), with the values of a tile in flight while
+// the digits are looked up.  Four blocks of 64 registers (three with 8-byte keys) that
+// read the values when they need them took longer above a million pairs, and above 4M
+// longer than tiles without a ticket loop; three of 85 gain 3 to 8 % from 8M on and lose
+// 6 to 15 % between.  Three passes of 32-bit pairs by two, three and four blocks
+// (us): 1M 93, 93 and 112; 2M 145, 165 and 158; 4M 231, 237 and 266; 16M 796, 749 and 878;
+// eight of 64-bit Morton codes: 1M 184 and (three) 217; 4M 485 and 603; 16M 1,656
+// and 1,948.
+constexpr int kSweepBlocks = 2;
 // Lanes of vmask with this lane's digit.  A match takes a turn per distinct
 // digit, a vote per bit eight turns always.  The 64-bit keys are Morton codes,
 // whose low digits are random: 1M pairs, eight passes, 244 us with matches and 214
 // with votes.  The 32-bit keys have few distinct digits in a warp in most sorts:
-// 8M pairs of 37 different keys 342 us with matches and 472 with votes.
-template <class K>
+// 8M pairs of 37 different keys 342 us with matches and 472 with votes.  Large
+// sorts of 64-bit keys look for a single digit first, as the high ones of equal or
+// neighbouring codes are: 4M pairs of 40 different keys 594 us without, 490 so,
+// of random ones 601 and 610; small ones lose 6 % by it.
+template <class K, int kN>
 __device__ __forceinline__ uint32_t same_digit(uint32_t vmask, uint32_t dig) {
     if constexpr (sizeof(K) == 4) return __match_any_sync(vmask, dig);
+    if constexpr (kN == kItems) {
+        int all;
+        __match_all_sync(vmask, dig, &all);
+        if (all) return vmask;
+    }
     uint32_t peers = vmask;
 #pragma unroll
     for (int b = 0; b < 8; b++) {
@@ -283,7 +297,7 @@ __device__ __forceinline__ void sweep_tiles(
             uint32_t vmask = __ballot_sync(0xFFFFFFFFu, ok);
             if (ok) {
                 const uint32_t dig = digit_of(key[i], bit, mask, desc != 0);
-                const uint32_t peers = same_digit<K>(vmask, dig);
+                const uint32_t peers = same_digit<K, kN>(vmask, dig);
                 uint32_t prior = wh[dig];
                 __syncwarp(vmask);
                 if (lane == (__ffs(peers) - 1)) wh[dig] = prior + __popc(peers);
@@ -293,15 +307,12 @@ __device__ __forceinline__ void sweep_tiles(
         }
         __syncthreads();
 
-        // the values: in flight during the look-back where registers are left
-        constexpr bool kEarly = kN <= kMidItems;
-        uint32_t val[kEarly ? kN : 1];
-        if constexpr (kEarly) {
+        // the values: in flight during the look-back
+        uint32_t val[kN];
 #pragma unroll
-            for (int i = 0; i < kN; i++) {
-                const uint32_t idx = wbase + i * 32 + lane;
-                val[i] = valsIn ? (idx < n ? valsIn[idx] : 0u) : idx;
-            }
+        for (int i = 0; i < kN; i++) {
+            const uint32_t idx = wbase + i * 32 + lane;
+            val[i] = valsIn ? (idx < n ? valsIn[idx] : 0u) : idx;
         }
         // ---- per digit: warp prefix, tile count, look-back ----
         {
@@ -364,8 +375,7 @@ __device__ __forceinline__ void sweep_tiles(
                 const uint32_t dig = place[i] >> 16;
                 uint32_t p = sm.digitStart[dig] + sm.warpHist[warp][dig] + (place[i] & 0xFFFFu);
                 sm.keys[p] = key[i];
-                if constexpr (kEarly) sm.vals[p] = val[i];
-                else sm.vals[p] = valsIn ? valsIn[idx] : idx;
+                sm.vals[p] = val[i];
             }
         }
         __syncthreads();
@@ -382,7 +392,7 @@ __device__ __forceinline__ void sweep_tiles(
 }
 
 template <class K, bool kDense>
-__global__ void __launch_bounds__(kThreads, kSweepBlocks<K>) k_onesweep(
+__global__ void __launch_bounds__(kThreads, kSweepBlocks) k_onesweep(
     const K* __restrict__ keysIn, K* __restrict__ keysOut, const uint32_t* __restrict__ valsIn,
     uint32_t* __restrict__ valsOut, const uint32_t* __restrict__ dCount, uint32_t hCount,
     const uint32_t* __restrict__ hist, uint32_t* tileStatus, uint32_t* tileTicket, int bit,
@@ -480,7 +490,7 @@ int sort_impl(const K* srcKeys, const uint32_t* srcVals, K* dstKeys, uint32_t* d
         srcKeys, dCount, maxCount, beginBit, endBit, desc ? 1 : 0, hist, status, epochs ? 1 : 0, P);
     // as many blocks as run at once; each takes tiles until they are used up,
     // so a small count on the device costs no blocks that only look for work
-    const uint32_t grid = std::min(tiles, 148u * uint32_t(kSweepBlocks<K>));
+    const uint32_t grid = std::min(tiles, 148u * uint32_t(kSweepBlocks));
     const K* kin = srcKeys;
     const uint32_t* vin = srcVals;
     for (int pass = 0; pass < passes && maxCount > 0; pass++) {
