@@ -1210,7 +1210,11 @@ int mrb_accel_construct(mrb_scene* s, void* stream) {
         // everything that lives only through the build comes out of one
         // allocation: the PLOC tree and its scratch, the collapse's, the probes'
         auto part = [](size_t bytes) { return (bytes + 255) & ~size_t(255); };
-        const size_t collapse = part(std::max(wide_scratch_bytes(n), wide_probe_bytes()));
+        // (the probes' 3.4 MB only where they run: an allocation of megabytes
+        // costs half a millisecond, several times the build of a small scene)
+        const bool probes = s->wideCollapse == 2 || s->wideOrderMode == MRB_WIDE_AUTO;
+        const size_t collapse =
+            part(std::max(wide_scratch_bytes(n), probes ? wide_probe_bytes() : size_t(0)));
         const bool ploc = s->wideTree != 0;
         const PlocArrays pa = ploc_arrays(n);
         DBuf temp;
