@@ -70,13 +70,18 @@ int trace_closest_wide(const WideAccelDev& acc, const float4* rayO, const float4
 // The most rays that a warp each traces faster than a lane each, by the scene's
 // triangles.  A launch of lanes lasts as long as its longest ray, the longer the more
 // levels the tree has, and hardly longer for more rays; the warps' work grows with the
-// rays, about a microsecond per thousand.  Camera rays or random ones, whichever
-// gains less, warps and the fastest lanes (us): 12 triangles, 4,096 rays 5.2 and 5.1,
-// 8,192 6.4 and 5.1; 100, 8,192 8.5 and 10.4, 12,288 10.0 and 8.5; 396, 16,384 18.7
-// and 20.8, 24,576 25.8 and 23.2; 2,316, 24,576 28.2 and 31.0, 32,768 36.1 and 28.9; 5,000 and more,
-// 32,768 37.2 and 37.1 to 88.6 and 106.7; 1M, 65,536 the same.
+// rays, about a microsecond per thousand.  Warps and the fastest lanes (us), the less
+// favourable of camera and random rays: 12 triangles, 4,096 rays 5.2 and 5.1, 8,192 6.4 and
+// 5.1; 100, 8,192 8.5 and 8.5, 12,288 10.0 and 8.5; 396, 16,384 18.7 and 20.8, 24,576
+// 25.8 and 23.2; 1,000, 24,576 22.7 and 22.6, 32,768 27.4 and 22.7; 2,316, 24,576 28.2 and 31.0,
+// 32,768 36.1 and 28.9; 3,000, 32,768 37.2 and 37.1; 1M, 32,768 88.6 and 106.7, 65,536
+// the same.
 inline uint32_t wide_warp_rays(uint32_t triangles) {
-    return triangles < 64 ? 4096 : triangles < 256 ? 8192 : triangles < 4096 ? 16384 : 32768;
+    return triangles < 64     ? 4096
+           : triangles < 256  ? 8192
+           : triangles < 900  ? 16384
+           : triangles < 3000 ? 24576
+                              : 32768;
 }
 // The same closest hits by a warp per ray (two triangles or more).
 int trace_closest_wide_few(const WideAccelDev& acc, const float4* rayO, const float4* rayD,

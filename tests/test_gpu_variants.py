@@ -414,12 +414,12 @@ def test_shadow_rays_see_what_the_binary_traversal_sees(system, cuda, order, shi
 
 
 # ---- few rays ----------------------------------------------------------------
-# the lines are at 4,096 rays below 64 triangles, 8,192 below 256, 16,384 below
-# 4,096, and 32,768
+# the lines are at 4,096 rays below 64 triangles, 8,192 below 256, 16,384 below 900,
+# 24,576 below 3,000, and 32,768
 @pytest.mark.parametrize("name,n", [
     *((s, n) for s in ("clusters", "cornell") for n in (1, 3, 4, 5, 2000, 32767, 32768, 32769)),
     *((s, n) for s in (2, 63) for n in (1, 4096, 4097)), (64, 8192), (255, 8193), (256, 16384),
-    (4095, 16385), (4096, 32768)])
+    (899, 16385), (900, 24576), (2999, 24577), (3000, 32768)])
 def test_few_rays_hit_what_a_lane_per_ray_hits(system, cuda, name, n):
     """Up to 32,768 rays, fewer over small scenes, a warp traces each ray, with the
     same triangle test: the distances are the same bits, and the triangles too but
