@@ -217,7 +217,7 @@ __global__ void __launch_bounds__(kInferThreads, 4) k_mlp_infer(MlpDev m,
         }
         __syncthreads();
     }
-    // a block without a tile, or one that gave up, still owns its copy
+    // a block without a tile still owns its copy
     if (first && ok) weights_wait(S, m.errorFlag);
     mlp_epilogue(S, S.tmem, 64);
 }

@@ -83,7 +83,7 @@ __device__ __forceinline__ void mbar_init(uint64_t* mbar, uint32_t count) {
                  : "memory");
 }
 
-// The error word may lie in mapped host memory: a plain store.
+// A plain store: every writer writes 1, and the word is read after the kernel.
 __device__ __forceinline__ void set_flag(uint32_t* flag) {
     *reinterpret_cast<volatile uint32_t*>(flag) = 1u;
 }
