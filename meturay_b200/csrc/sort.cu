@@ -210,12 +210,13 @@ __device__ __forceinline__ void block_exclusive2(uint32_t a, uint32_t b, uint32_
 constexpr int kSweepBlocks = 2;
 // Lanes of vmask with this lane's digit.  A match takes a turn per distinct
 // digit, a vote per bit eight turns always.  The 64-bit keys are Morton codes,
-// whose low digits are random: 1M pairs, eight passes, 244 us with matches and 214
-// with votes.  The 32-bit keys have few distinct digits in a warp in most sorts:
-// 8M pairs of 37 different keys 342 us with matches and 472 with votes.  Large
+// whose low digits are random: 1M pairs, eight passes, 206 us with matches and 184
+// with votes, 4M 572 and 488.  The 32-bit keys are mostly a wavefront's materials, few
+// distinct ones: 4M pairs of 2 to 12 different keys, two passes, 98 to 102 us with
+// matches and 110 with votes; of 40 113 and 111, of random ones 153 and 129.  Large
 // sorts of 64-bit keys look for a single digit first, as the high ones of equal or
-// neighbouring codes are: 4M pairs of 40 different keys 594 us without, 490 so,
-// of random ones 601 and 610; small ones lose 6 % by it.
+// neighbouring codes are (at three blocks per SM, 4M pairs of 40 different keys 594 us
+// without, 490 so, of random ones 601 and 610); small ones lose 6 % by it.
 template <class K, int kN>
 __device__ __forceinline__ uint32_t same_digit(uint32_t vmask, uint32_t dig) {
     if constexpr (sizeof(K) == 4) return __match_any_sync(vmask, dig);
@@ -245,7 +246,8 @@ __device__ __forceinline__ void sweep_tiles(
     const uint32_t ltMask = (1u << lane) - 1u;
     const uint32_t tiles = tile_count(n);
     // more blocks than tiles would crowd the tiles on the SMs that start first
-    // (480 blocks for 245 tiles of a million pairs: 128 us, 99 us so)
+    // (at four blocks per SM, 480 blocks for 245 tiles of a million pairs: 128 us,
+    // 99 us so)
     if (blockIdx.x >= tiles) return;
     for (;;) {
         if (tid == 0) sm.tile = atomicAdd(tileTicket, 1u);
